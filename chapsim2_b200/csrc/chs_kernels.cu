@@ -743,6 +743,14 @@ void launch_line_op_t(int d, const OpPlan& P, const LineIOT<T>& io, const double
     else launch_stencil_dir<T, 2>(P, io, table, st, nlines);
     return;
   }
+  // lines in register pieces (chs_line.cu; 32-bit indices); the tile kernel keeps lines of more than
+  // 384 points and the collocated families D1C2C and D1P2P, which no substep uses.  CP6 128x96x128
+  // line solves of a substep: 486 us in pieces, 1029 us by the tile kernel
+  const int64_t total = nl * (P.nin > P.nout ? P.nin : P.nout);
+  if (P.lrows && total + 32 * 512 < 0x7fffffff) {
+    launch_line_chunk<T>(d, P, io, table, st, nlines);
+    return;
+  }
   const int nmax = P.nin > P.nout ? P.nin : P.nout;
   // up to 64 lines per CTA, fewer while the tile exceeds ~45 KB so that four or more CTAs
   // (32+ warps) stay resident per SM

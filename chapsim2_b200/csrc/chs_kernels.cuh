@@ -54,6 +54,11 @@ using LineIO = LineIOT<double>;
 void launch_line_op(int d, const OpPlan& plan, const LineIO& io, const double* table, cudaStream_t st);
 void launch_line_op(int d, const OpPlan& plan, const LineIOT<float>& io, const double* table, cudaStream_t st);
 
+// compact plan with lrows > 0 as register pieces (chs_line.cu)
+template <typename T>
+void launch_line_chunk(int d, const OpPlan& P, const LineIOT<T>& io, const double* table, cudaStream_t st,
+                       int nlines);
+
 // nondimensional property table on the device, sorted by T (FP64 columns)
 struct ThermoTab {
   const double *t, *h, *d, *m, *k, *rhoh;

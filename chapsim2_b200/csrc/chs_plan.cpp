@@ -562,6 +562,36 @@ void thomas(std::vector<double>& x, const std::vector<double>& a, const std::vec
 
 }  // namespace
 
+// whether the plan's boundary rows are its bulk formula with wrapped indices, term by term
+static bool wrapped_bulk(const OpPlan& p) {
+  int o[4];
+  double cf[4];
+  const double r1 = p.r1, r2 = p.r2;
+  switch (p.fam) {
+    case M1P2C: o[0] = 0; o[1] = 1; o[2] = -1; o[3] = 2; cf[0] = r1; cf[1] = r1; cf[2] = r2; cf[3] = r2; break;
+    case M1C2P: o[0] = 0; o[1] = -1; o[2] = 1; o[3] = -2; cf[0] = r1; cf[1] = r1; cf[2] = r2; cf[3] = r2; break;
+    case D1C2C:
+    case D1P2P: o[0] = 1; o[1] = -1; o[2] = 2; o[3] = -2; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
+    case D1C2P: o[0] = 0; o[1] = -1; o[2] = 1; o[3] = -2; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
+    default: o[0] = 1; o[1] = 0; o[2] = 2; o[3] = -1; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
+  }
+  const int n = p.nin;
+  const double tol = 1e-13 * (std::fabs(r1) + std::fabs(r2));
+  int covered = 0;
+  for (int s = 0; s < p.nspec; ++s) {
+    const SpecialRow& S = p.sp[s];
+    for (int u = 0; u < 4; ++u)
+      if (S.wb[u] != 0.0) return false;
+    std::vector<double> want(n, 0.0), have(n, 0.0);
+    for (int k = 0; k < 4; ++k) want[((S.row + o[k]) % n + n) % n] += cf[k];
+    for (int t = 0; t < S.nt; ++t) have[S.idx[t]] += S.w[t];
+    for (int i = 0; i < n; ++i)
+      if (std::fabs(want[i] - have[i]) > tol) return false;
+    if (S.row < p.b_lo || S.row > p.b_hi) ++covered;
+  }
+  return covered == p.b_lo + (p.nout - 1 - p.b_hi);
+}
+
 void reduce_bc(int fam, const int ibc0[2], bool has_fbc, int ibc[2]) {
   for (int k = 0; k < 2; ++k) {
     ibc[k] = ibc0[k];
@@ -694,41 +724,44 @@ OpPlan PlanBook::make(int d, int fam, const int ibc0[2], bool has_fbc) {
       if (p.neu1 || p.neu2) p.needs_fbc = 1;
     }
   }
-  // A periodic explicit line whose boundary rows equal the bulk stencil with wrapped indices runs
-  // every row through the bulk formula (no per-row branches in the kernels).  The check compares
-  // the assembled boundary rows with the kernels' bulk formula term by term.
-  p.wrap = 0;
-  if (p.tdma == 0 && ibc[0] == BC_PERIODIC && ibc[1] == BC_PERIODIC && p.nin == p.nout && p.lmap < 0 && !p.neu1 &&
-      !p.neu2) {
-    int o[4];
-    double cf[4];
-    const double r1 = p.r1, r2 = p.r2;
-    switch (fam) {
-      case M1P2C: o[0] = 0; o[1] = 1; o[2] = -1; o[3] = 2; cf[0] = r1; cf[1] = r1; cf[2] = r2; cf[3] = r2; break;
-      case M1C2P: o[0] = 0; o[1] = -1; o[2] = 1; o[3] = -2; cf[0] = r1; cf[1] = r1; cf[2] = r2; cf[3] = r2; break;
-      case D1C2C:
-      case D1P2P: o[0] = 1; o[1] = -1; o[2] = 2; o[3] = -2; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
-      case D1C2P: o[0] = 0; o[1] = -1; o[2] = 1; o[3] = -2; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
-      default: o[0] = 1; o[1] = 0; o[2] = 2; o[3] = -1; cf[0] = r1; cf[1] = -r1; cf[2] = r2; cf[3] = -r2; break;
-    }
-    const int n = p.nin;
-    const double tol = 1e-13 * (std::fabs(r1) + std::fabs(r2));
-    bool ok = true;
-    int covered = 0;
-    for (int s = 0; s < p.nspec && ok; ++s) {
-      const SpecialRow& S = p.sp[s];
-      for (int u = 0; u < 4; ++u)
-        if (S.wb[u] != 0.0) ok = false;
-      std::vector<double> want(n, 0.0), have(n, 0.0);
-      for (int k = 0; k < 4; ++k) want[((S.row + o[k]) % n + n) % n] += cf[k];
-      for (int t = 0; t < S.nt; ++t) have[S.idx[t]] += S.w[t];
-      for (int i = 0; i < n && ok; ++i)
-        if (std::fabs(want[i] - have[i]) > tol) ok = false;
-      if (S.row < p.b_lo || S.row > p.b_hi) ++covered;
-    }
-    if (ok && covered == p.b_lo + (p.nout - 1 - p.b_hi)) p.wrap = 1;
-  }
+  // A periodic line whose boundary rows equal the bulk stencil with wrapped indices runs every row
+  // through the bulk formula (no per-row branches in the kernels).
+  const bool per = ibc[0] == BC_PERIODIC && ibc[1] == BC_PERIODIC && p.nin == p.nout && !p.neu1 && !p.neu2 &&
+                   wrapped_bulk(p);
+  p.wrap = per && p.tdma == 0 && p.lmap < 0;
+  p.lwrap = per && p.tdma == 2;
+  p.lrows = 0;
+  p.lcoef = p.lcoef32 = -1;
+  if (p.tdma && fam != D1C2C && fam != D1P2P) line_coefs(p);
   return p;
+}
+
+// Row factors of a compact line cut into pieces of lrows rows (chs_line.cu): D = 1/pivot, A = a D, P
+// and Q the products of -A (-C) from the piece's start (to its end), C = c/pivot, X the cyclic
+// correction, M the metric.  Rows past the end are zero; the last row of a periodic line, which is
+// not part of the Thomas system, passes its right-hand side through.
+void PlanBook::line_coefs(OpPlan& p) {
+  const int n = p.nout, R = line_piece_rows(std::max(p.nin, p.nout));
+  if (R == 0) return;
+  const int nsw = p.tdma == 2 ? n - 1 : n, rows = (std::max(p.nin, n) + R - 1) / R * R;
+  std::vector<double> f((size_t)rows * kLineCoefs, 0.0);
+  auto at = [&](int i, int k) -> double& { return f[(size_t)i * kLineCoefs + k]; };
+  for (int i = 0; i < n; ++i) {
+    const bool in = i < nsw;
+    at(i, 0) = !in ? 1.0 : (i == 0 ? 1.0 / p.b1 : table[p.ld + i]);
+    at(i, 1) = in && i > 0 ? table[p.la + i] * table[p.ld + i] : 0.0;
+    at(i, 3) = i < nsw - 1 ? table[p.lc + i] : 0.0;
+    at(i, 5) = p.tdma == 2 && in ? table[p.lx1 + i] : 0.0;
+    at(i, 6) = p.lmap >= 0 ? table[p.lmap + i] : 1.0;
+  }
+  for (int i = 0; i < rows; ++i) at(i, 2) = -at(i, 1) * (i % R == 0 ? 1.0 : at(i - 1, 2));
+  for (int i = rows - 1; i >= 0; --i) at(i, 4) = -at(i, 3) * (i % R == R - 1 ? 1.0 : at(i + 1, 4));
+  std::vector<float> f32(f.begin(), f.end());
+  std::vector<double> packed(f.size() / 2);
+  std::memcpy(packed.data(), f32.data(), f32.size() * sizeof(float));
+  p.lcoef = add_array(f);
+  p.lcoef32 = add_array(packed);
+  p.lrows = R;
 }
 
 }  // namespace chs

@@ -62,9 +62,25 @@ struct OpPlan {
   int64_t lmap;          // y-mapping multiplier (nout) or -1
   int neu1, neu2;        // overwrite first/last row with fbc(1)/fbc(2)
   int needs_fbc;         // 1 if any boundary value is read
+  // compact lines in register pieces (chs_line.cu): rows per thread (0: the line has no such form),
+  // offsets of the row factors in FP64 and, packed two to a double, in FP32; lwrap: a periodic line
+  // whose boundary rows are the bulk stencil with wrapped indices
+  int lrows, lwrap;
+  int64_t lcoef, lcoef32;
   int wrap;              // periodic explicit line whose boundary rows are the bulk stencil with
                          // wrapped indices: every row may use the bulk formula
 };
+
+// Pieces of a compact line: at most kLineWarps of them (one warp each, 32 lines side by side), of 8
+// rows up to 128 points, 16 up to 256 and 24 up to 384; longer lines run line_op_kernel.  kLineCoefs
+// factors per row.
+constexpr int kLineWarps = 16;
+constexpr int kLineCoefs = 8;
+inline int line_piece_rows(int n) {
+  for (int r = 8; r <= 24; r += 8)
+    if (n <= r * kLineWarps) return r;
+  return 0;
+}
 
 // Builds plans and the LHS/mapping table they reference.
 class PlanBook {
@@ -89,6 +105,7 @@ class PlanBook {
   struct LhsKey { int fam, n, b1, b2; int64_t la, lc, ld, lx1; double b1v, an, cn, inv_den; };
   std::vector<LhsKey> lhs_;
   const LhsKey& lhs(int fam, int n, int bc1, int bc2);
+  void line_coefs(OpPlan& p);
 };
 
 void reduce_bc(int fam, const int ibc0[2], bool has_fbc, int ibc[2]);
