@@ -244,16 +244,16 @@ struct FzCtx {
     return TH ? v * muyz(i, j, k) : v;
   }
 
-  // the fractional step of the operator path's O_FRAC store (pfc = 1 * v); last = m0[c][a], loaded
-  // by the caller before the stencil loads so that no load waits behind the stores
-  __device__ __forceinline__ T frac(int c, int a, T F, T v, T last) const {
+  // the fractional step of the operator path's O_FRAC store (pfc = 1 * v); last = m0[c][a] and own, the
+  // advanced field, loaded by the caller before the stencil loads so that no load waits behind the stores
+  __device__ __forceinline__ T frac(int c, int a, T F, T v, T last, T own) const {
     const T tdt = T(f.dt), tg = T(f.gam), tz = T(f.zeta), ta = T(f.alpha);
     const T pfc = T(1.0) * v;
     T tot = tg * F + tz * last;
     f.m0[c][a] = F;
     tot = tot + ta * pfc;
     const T r = tdt * tot;
-    f.m[c][a] = r;
+    f.m[c][a] = f.adv >> c & 1 ? own + r : r;
     return r;
   }
 };
@@ -267,6 +267,7 @@ __device__ __forceinline__ T fz_momentum_body(const FzMomentum<T>& f, int i, int
   const double r = f.rre;
   const int a = (k * (C == 1 ? np1 : nc1) + j) * n0 + i;
   const T last = f.m0[C][a];
+  const T own = TH ? (C == 0 ? f.gx : C == 1 ? f.gy : f.gz)[a] : (C == 0 ? f.qx : C == 1 ? f.qy : f.qz)[a];
   T F, v;
   if (C == 0) {
     // x-momentum at (i, j, k) of the qx grid
@@ -280,7 +281,7 @@ __device__ __forceinline__ T fz_momentum_body(const FzMomentum<T>& f, int i, int
         f.term[0][2], f.rows, nl, n0, i, j, k, n2, 1.0, r, [&](int q) { return c.template conv_xz<0>(i, j, q); },
         [&](double s, int q) { return c.visc_xz(s, i, j, q); });
     v = fz_per<D1C2P, T, WX>(f.pres[0], i, n0, [&](int q) { return T(-1.0) * c.pr(q, j, k); });
-    return c.frac(0, a, F, v, last);
+    return c.frac(0, a, F, v, last, own);
   } else if (C == 1) {
     // y-momentum at (i, j, k) of the qy grid
     F = fz_pair<D1P2C, 0, PY, E, T, WX, WZ>(
@@ -294,7 +295,7 @@ __device__ __forceinline__ T fz_momentum_body(const FzMomentum<T>& f, int i, int
         [&](double s, int q) { return c.visc_yz(s, i, j, q); });
     v = fz_y<D1C2P, PY, E, T>(f.rows, f.pres[1], j, nc1, f.fpres[1], nl, L,
                            [&](int q) { return T(-1.0) * c.pr(i, q, k); });
-    return c.frac(1, a, F, v, last);
+    return c.frac(1, a, F, v, last, own);
   } else {
     // z-momentum at (i, j, k) of the qz grid
     F = fz_pair<D1P2C, 0, PY, E, T, WX, WZ>(
@@ -307,7 +308,7 @@ __device__ __forceinline__ T fz_momentum_body(const FzMomentum<T>& f, int i, int
         f.term[2][2], f.rows, nl, n0, i, j, k, n2, 2.0, r, [&](int q) { return c.template conv_c<2>(i, j, q); },
         [&](double s, int q) { return c.template visc_c<2>(s, i, j, q); });
     v = fz_per<D1C2P, T, WZ>(f.pres[2], k, n2, [&](int q) { return T(-1.0) * c.pr(i, j, q); });
-    return c.frac(2, a, F, v, last);
+    return c.frac(2, a, F, v, last, own);
   }
 }
 
@@ -381,6 +382,15 @@ __global__ void fz_wall_visc_kernel(const __grid_constant__ FzMomentum<T> f, T* 
       }
     }
   }
+}
+
+// the wall rows of the y component, beside the march that forms the others (chs_march.cu)
+template <typename T, bool TH>
+__global__ void fz_wall_rows_kernel(const __grid_constant__ FzMomentum<T> f) {
+  const int nl = f.n0 * f.n2, gs = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gs >= 2 * nl) return;
+  const int side = gs < nl ? 0 : 1, g = gs - side * nl, k = g / f.n0;
+  fz_momentum_body<T, TH, false, 1, true>(f, g - k * f.n0, side == 0 ? 0 : f.np1 - 1, k);
 }
 
 template <typename T>
@@ -585,16 +595,15 @@ __global__ void __launch_bounds__(256) fz_project_kernel(const __grid_constant__
   const T cf = T(f.coef);
   // every read-modify-write value is loaded before the first store, so that no load waits behind one
   const int b = (k * np1 + j) * n0 + i;
-  T uy0 = f.uy[b];
-  if (f.upd) uy0 = uy0 + (f.my[b] - T(0));
+  const T uy0 = (f.upd ? f.my : f.uy)[b];
   if (j < nc1) {
     const int a = (k * nc1 + j) * n0 + i;
     const T p0 = f.p[a];
-    T ux0 = f.ux[a], uz0 = f.uz[a];
+    const T uz0 = (f.upd ? f.mz : f.uz)[a];
+    T ux0 = f.ux[a];
     if (f.upd) {
       const T s = f.bulk ? T(f.bulk[0]) : T(0);
-      ux0 = ux0 + (f.mx[a] - s);
-      uz0 = uz0 + (f.mz[a] - T(0));
+      ux0 = f.upd == 2 ? ux0 + (f.mx[a] - s) : f.mx[a] - s;
     }
     // p += phi (axpby with unit weights)
     T pv = T(1.0) * p0;
@@ -624,7 +633,7 @@ __global__ void __launch_bounds__(256) fz_project_kernel(const __grid_constant__
   }
 }
 
-// ---- momentum advance folded into the Poisson right-hand side: thread per cell (i, j, k)
+// ---- Poisson right-hand side of the advanced fields: thread per cell (i, j, k)
 template <typename T>
 __global__ void __launch_bounds__(256) fz_update_div_kernel(const __grid_constant__ FzUpdateDiv<T> f) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -633,22 +642,19 @@ __global__ void __launch_bounds__(256) fz_update_div_kernel(const __grid_constan
   const int n0 = f.n0, nc1 = f.nc1, np1 = f.np1, n2 = f.n2;
   if (i >= n0 || j >= nc1 || k >= n2) return;
   const T s = f.bulk ? T(f.bulk[0]) : T(0);
-  // u' at a face (fz_update_kernel's arithmetic)
+  // u' at a face
   auto gx = [&](int q) {
     const int a = (k * nc1 + j) * n0 + q;
-    return __ldg(f.ux + a) + (__ldg(f.mx + a) - s);
+    return f.mx ? __ldg(f.ux + a) + (__ldg(f.mx + a) - s) : __ldg(f.ux + a) - s;
   };
   auto gy = [&](int q) {
     const int b = (k * np1 + q) * n0 + i;
-    T v = __ldg(f.uy + b) + (__ldg(f.my + b) - T(0));
+    T v = __ldg(f.uy + b);
     if (f.s0 && q == 0) v = T(f.v0);
     if (f.s1 && q == np1 - 1) v = T(f.v1);
     return v;
   };
-  auto gz = [&](int q) {
-    const int a = (q * nc1 + j) * n0 + i;
-    return __ldg(f.uz + a) + (__ldg(f.mz + a) - T(0));
-  };
+  auto gz = [&](int q) { return __ldg(f.uz + (q * nc1 + j) * n0 + i); };
   const T vx = fz_per<D1P2C, T>(f.dx, i, n0, gx);
   const T vy = fz_row<T>(f.rows, f.dy, j, f.fdy, n0 * n2, i + n0 * k, gy);
   const T vz = fz_per<D1P2C, T>(f.dz, k, n2, gz);
@@ -720,6 +726,13 @@ void launch_fz_wall_visc(const FzMomentum<T>& f, T* fvisc2, T* fcomb, const T* f
 }
 
 template <typename T>
+void launch_fz_wall_rows(const FzMomentum<T>& f, cudaStream_t st) {
+  const int blocks = (2 * f.n0 * f.n2 + 127) / 128;
+  if (f.thermo) fz_wall_rows_kernel<T, true><<<blocks, 128, 0, st>>>(f);
+  else fz_wall_rows_kernel<T, false><<<blocks, 128, 0, st>>>(f);
+}
+
+template <typename T>
 void launch_fz_update(T* ux, T* uy, T* uz, const T* mx, const T* my, const T* mz, const double* bulk, int n0,
                       int nc1, int np1, int n2, int s0, double v0, int s1, double v1, cudaStream_t st) {
   const dim3 grid((n0 + 127) / 128, np1, n2);
@@ -758,6 +771,8 @@ template void launch_fz_momentum<double>(const FzMomentum<double>&, int, cudaStr
 template void launch_fz_momentum<float>(const FzMomentum<float>&, int, cudaStream_t);
 template void launch_fz_wall_visc<double>(const FzMomentum<double>&, double*, double*, const double*, cudaStream_t);
 template void launch_fz_wall_visc<float>(const FzMomentum<float>&, float*, float*, const float*, cudaStream_t);
+template void launch_fz_wall_rows<double>(const FzMomentum<double>&, cudaStream_t);
+template void launch_fz_wall_rows<float>(const FzMomentum<float>&, cudaStream_t);
 template void launch_fz_update<double>(double*, double*, double*, const double*, const double*, const double*,
                                        const double*, int, int, int, int, int, double, int, double, cudaStream_t);
 template void launch_fz_update<float>(float*, float*, float*, const float*, const float*, const float*,

@@ -75,7 +75,9 @@ struct FzMomentum {
   FzPair<T> term[3][3];  // [component][direction]
   FzOp pres[3];          // pressure gradient of each component
   const T* fpres[3];
-  T *m[3], *m0[3];       // right-hand sides (fractional-step increments) and their histories
+  T *m[3], *m0[3];       // increments m of the fractional step, or advanced fields u + m where bit c of
+                         // adv is set (u the momentum g with variable properties, else q); histories
+  int adv;
   double rre, dt, gam, zeta, alpha;
   const FzRow* rows;     // row tables of the y operators
   // constant mass flux: the x component also writes, per CTA, the y-weighted sum of its outputs
@@ -84,10 +86,39 @@ struct FzMomentum {
   double* part;
 };
 
+// ---- the three momentum components in one pass (chs_march.cu), for the operators the host has found to
+// be the plain staggered second-order ones: x and z periodic with weights 1/2 and 1/h; y periodic, or
+// with walls whose interior rows are two-point with weights 1/2, wc[j] (points to cells) and wp[j] (cells
+// to points) and whose wall rows are the wall plane's value and twice the one-sided difference to it.
+// Wall rows of the y component are left to launch_fz_wall_rows.
+template <typename T>
+struct FzMarch {
+  int n0, nc1, np1, n2;
+  const T* a[8];                   // qx, qy, qz, p; with variable properties gx, gy, gz, mu
+  const T *bqx, *bqz, *bg, *bmu;   // wall planes (below, above) of qx, qz, the momentum and mu
+  const double *wc, *wp;           // y weights of the cells and the points
+  double dxi, dzi;                 // 1/h in x and z
+  double rre, dt, gam, zeta, alpha;
+  T *out[3], *m0[3];               // increments m, or advanced fields u + m where bit c of adv is set; histories
+  int adv;
+  // constant mass flux: bulk[0] = sum(wy[j] m_x) / vol, through per-CTA sums (part, as long as
+  // fz_march_blocks_max) and a CTA counter that is zero between launches; part null otherwise
+  const double* wy;
+  double* part;
+  unsigned* count;
+  double* bulk;
+  double vol;
+  int chunk;                       // z planes per CTA (set by the launch)
+};
+template <typename T>
+void launch_fz_march(const FzMarch<T>& f, bool thermo, bool periodic_y, cudaStream_t st);
+int fz_march_blocks_max(int n0, int ny, int n2);
+
 // bulk[0] = (sum of the x pass's nblk per-CTA sums) / vol, in a fixed order (one CTA)
 void launch_fz_finalize_mean(const double* part, int nblk, double* bulk, double vol, cudaStream_t st);
 // the right-hand side of momentum component c (0 x, 1 y, 2 z) with the fractional step
-// (m = dt*(gam*F + zeta*m0 + alpha*pfc), m0 = F); the advance q += m is left to launch_fz_update
+// (m = dt*(gam*F + zeta*m0 + alpha*pfc), m0 = F); without adv the advance q += m is left to
+// launch_fz_update
 template <typename T>
 void launch_fz_momentum(const FzMomentum<T>& f, int c, cudaStream_t st);
 // CTAs of the x component's launch (the length of f.part)
@@ -98,6 +129,10 @@ int fz_momentum_x_blocks(int n0, int nc1, int n2);
 // each side into planes side and side + 2
 template <typename T>
 void launch_fz_wall_visc(const FzMomentum<T>& f, T* fvisc2, T* fcomb, const T* fconv2, cudaStream_t st);
+
+// the wall rows of the y component (launch_fz_momentum's rows 0 and np1 - 1 of component 1)
+template <typename T>
+void launch_fz_wall_rows(const FzMomentum<T>& f, cudaStream_t st);
 
 // q advance after the mass-flux mean: ux += mx - bulk, uy += my, uz += mz, then the y walls of uy
 // set to v0 / v1 (flags s0 / s1)
@@ -151,8 +186,8 @@ struct FzProject {
   int s0, s1;                     // y walls of uy set to v0 / v1
   double v0, v1;
   const FzRow* rows;
-  // upd: the advance of the momentum step (u += m - bulk, fz_update_kernel's arithmetic) is done
-  // here, at each thread's own point, before the correction (the momentum step left u unchanged)
+  // upd 1: the projection starts from the momentum step's advanced fields mx (less the mass-flux mean),
+  // my, mz, and u is written here only; 2: the same with mx the increment, u + (mx - bulk)
   int upd;
   const T *mx, *my, *mz;
   const double* bulk;
@@ -160,15 +195,15 @@ struct FzProject {
 template <typename T>
 void launch_fz_project(const FzProject<T>& f, cudaStream_t st);
 
-// Poisson right-hand side coeff * (d/dx ux' + d/dy uy' + d/dz uz') of the advanced fields
-// u' = u + m - bulk (y wall rows of uy' set to v0 / v1), formed at each face from u and m without
-// storing u' (the projection stores it): the divergence of the operator path (run_fused on
-// D1P2C of u') with the momentum advance folded in
+// Poisson right-hand side coeff * (d/dx ux' + d/dy uy' + d/dz uz') of the advanced fields of the momentum
+// step, u' = u with the mass-flux mean subtracted in x and the y wall rows of uy set to v0 / v1: the
+// divergence of the operator path (run_fused on D1P2C of u')
 template <typename T>
 struct FzUpdateDiv {
   int n0, nc1, np1, n2;
-  const T *ux, *uy, *uz, *mx, *my, *mz;
-  const double* bulk;  // mass-flux mean subtracted from mx, or null
+  const T *ux, *uy, *uz;
+  const T* mx;         // increment still to be added to ux, or null
+  const double* bulk;  // mass-flux mean, or null
   int s0, s1;
   double v0, v1;
   FzOp dx, dy, dz;     // D1P2C: x and z periodic, y a row table

@@ -129,7 +129,10 @@ struct chs_handle {
   // >= 0 while chs_profile_class captures a substep: launches of other kernel classes are left out
   int only_kind = -1;
   FzRow* fz_rows = nullptr;  // device row tables of the y operators (chs_fused.cuh)
-  double* fz_part = nullptr;  // per-CTA partial sums of the mass-flux mean from the fused x pass
+  std::vector<FzRow> fz_rows_host;
+  double* fz_part = nullptr;  // per-CTA partial sums of the mass-flux mean from the fused momentum pass
+  unsigned* fz_count = nullptr;  // CTAs of that pass that have finished (zero between launches)
+  double* fz_w = nullptr;     // y weights of the momentum march: np[1] points, then nc[1] cells
   // plan key -> first row of its table in fz_rows (-1: no table: periodic, or not representable)
   std::map<std::tuple<int, int, int, int, int>, int> fz_index;
   long long launches = 0;
@@ -836,6 +839,15 @@ void setup_host(chs_handle* H, const chs_config* c) {
   setup_book(H, c);
 }
 
+// y weights of a first difference at the points and of one at the cells (1/h and the y metric)
+std::vector<double> fz_march_weights(const chs_handle* H) {
+  const double dd = 1.0 / H->h[1];
+  std::vector<double> w;
+  for (int j = 0; j < H->np[1]; ++j) w.push_back(dd * (H->stretch_y ? H->mppt[j] : 1.0));
+  for (int j = 0; j < H->nc[1]; ++j) w.push_back(dd * (H->stretch_y ? H->mpcc[j] : 1.0));
+  return w;
+}
+
 // device buffers and Poisson tables
 void setup_device(chs_handle* H, const chs_config* c) {
   const int nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2], np1 = H->np[1];
@@ -906,7 +918,11 @@ void setup_device(chs_handle* H, const chs_config* c) {
   CK(cudaMemcpyAsync(H->wy, wy.data(), nc1 * sizeof(double), cudaMemcpyHostToDevice, H->st));
   H->npart = 148 * 4;
   H->partial = H->dalloc<double>(2 * H->npart);
-  H->fz_part = H->dalloc<double>(fz_momentum_x_blocks(nc0, nc1, nc2));
+  H->fz_part = H->dalloc<double>(std::max(fz_momentum_x_blocks(nc0, nc1, nc2), fz_march_blocks_max(nc0, nc1, nc2)));
+  H->fz_count = H->dalloc<unsigned>(1);
+  H->fz_w = H->dalloc<double>(np1 + nc1);
+  const std::vector<double> fzw = fz_march_weights(H);
+  CK(cudaMemcpyAsync(H->fz_w, fzw.data(), fzw.size() * sizeof(double), cudaMemcpyHostToDevice, H->st));
   H->scal = H->dalloc<double>(16);
 
   // Poisson tables
@@ -1170,6 +1186,7 @@ void upload_fz_rows(chs_handle* H) {
     }
     H->fz_index[kv.first] = at;
   }
+  H->fz_rows_host = v;
   if (H->fz_rows) { CK(cudaFreeAsync(H->fz_rows, H->st)); H->fz_rows = nullptr; }
   if (v.empty()) v.push_back(FzRow{});  // periodic y: no tables, a valid pointer all the same
   CK(cudaMallocAsync(&H->fz_rows, v.size() * sizeof(FzRow), H->st));
@@ -1286,6 +1303,82 @@ struct FzBuild {
   }
 };
 
+// Whether the momentum pass may store the advanced x field u + m before the mass-flux mean is known, so
+// that u' = (u + m) - bulk.  Not in FP32 with a mean: the second rounding of values of the velocity's size
+// is a bias that 1000 steps of a laminar channel add up to 1.4e-5 of the mean profile (2e-6 with
+// u + (m - bulk)).
+template <typename T>
+bool advances_x(const chs_handle* H) {
+  return sizeof(T) == 8 || H->idriven != 1;
+}
+
+// Whether the momentum descriptor's operators are the plain staggered ones that the march along z
+// evaluates (FzMarch): every x and z operator two-point with weights 1/2 or 1/h, and every y operator
+// with walls so on its interior rows, with the wall plane's value, or twice the difference to it, on its
+// wall rows.  Symmetry and slope walls and odd nx keep the component kernels.
+template <typename T>
+bool fz_march_form(const chs_handle* H, const FzMomentum<T>& F) {
+  if (F.n0 % 2 || (int64_t)F.n0 * F.np1 * (F.n2 + 2) >= 0x7fffffff) return false;
+  const double dx = 1.0 / H->h[0], dz = 1.0 / H->h[2], dy = 1.0 / H->h[1];
+  const std::vector<double> wt = fz_march_weights(H);
+  const int ny = F.nc1, np1 = F.np1;
+  auto per = [](const FzOp& o, double w) { return o.row < 0 && o.r1 * o.dd == w; };
+  // row p of a wall operator: weights wh on input row h, wl on input row l, wall weight b of the row's side
+  auto row = [&](const FzOp& o, int p, int h, double wh, int l, double wl, double b0, double b1) {
+    const FzRow& r = H->fz_rows_host[o.row + p];
+    double a = 0.0, c = 0.0;
+    for (int t = 0; t < (r.flags & 1 ? 3 : 2); ++t) {
+      if (r.w[t] == 0.0) continue;
+      if (p + r.o[t] == h) a += r.w[t];
+      else if (p + r.o[t] == l) c += r.w[t];
+      else return false;
+    }
+    return a == wh && c == wl && (r.flags & 2 ? r.wb[0] : 0.0) == b0 && (r.flags & 4 ? r.wb[1] : 0.0) == b1;
+  };
+  // cells to points: interpolation (der 0) or derivative; walls: the wall rows too
+  auto c2p = [&](const FzOp& o, bool der, bool walls) {
+    if (F.periodic_y) return per(o, der ? dy : 0.5);
+    if (o.row < 0) return false;
+    for (int p = 1; p < np1 - 1; ++p)
+      if (!row(o, p, p, der ? wt[p] : 0.5, p - 1, der ? -wt[p] : 0.5, 0.0, 0.0)) return false;
+    if (!walls) return true;
+    if (!der) return row(o, 0, 0, 0.0, -1, 0.0, 1.0, 0.0) && row(o, ny, -1, 0.0, -1, 0.0, 0.0, 1.0);
+    return row(o, 0, 0, 2.0 * wt[0], -1, 0.0, -2.0 * wt[0], 0.0) &&
+           row(o, ny, ny - 1, -2.0 * wt[ny], -1, 0.0, 0.0, 2.0 * wt[ny]);
+  };
+  auto p2c = [&](const FzOp& o, bool der) {
+    if (F.periodic_y) return per(o, der ? dy : 0.5);
+    if (o.row < 0) return false;
+    for (int p = 0; p < ny; ++p)
+      if (!row(o, p, p + 1, der ? wt[np1 + p] : 0.5, p, der ? -wt[np1 + p] : 0.5, 0.0, 0.0)) return false;
+    return true;
+  };
+  auto in = [&](int s) -> const FzOp& { return F.in[s]; };
+  for (int s : {FI_QX_MX, FI_QX_MZ, FI_QY_MX, FI_QY_MZ, FI_QZ_MX, FI_QZ_MZ})
+    if (!per(in(s), 0.5)) return false;
+  for (int s : {FI_QX_DX, FI_QY_DX, FI_QZ_DX})
+    if (!per(in(s), dx)) return false;
+  for (int s : {FI_QX_DZ, FI_QY_DZ, FI_QZ_DZ})
+    if (!per(in(s), dz)) return false;
+  if (!c2p(in(FI_QX_DY), true, true) || !c2p(in(FI_QX_MY), false, true) || !c2p(in(FI_QZ_DY), true, true) ||
+      !c2p(in(FI_QZ_MY), false, true) || !p2c(in(FI_QY_DY), true) || !p2c(in(FI_QY_MY), false))
+    return false;
+  if (F.thermo) {
+    for (int s : {FI_GX_MX, FI_GX_MZ, FI_GY_MX, FI_GY_MZ, FI_GZ_MX, FI_GZ_MZ, FI_MU_YX, FI_MU_X, FI_MU_XZ, FI_MU_YZ})
+      if (!per(in(s), 0.5)) return false;
+    if (!c2p(in(FI_GX_MY), false, true) || !c2p(in(FI_GZ_MY), false, true) || !c2p(in(FI_MU_Y), false, true) ||
+        !p2c(in(FI_GY_MY), false))
+      return false;
+  }
+  for (int c = 0; c < 3; ++c)
+    for (int d = 0; d < 3; ++d)
+      for (int u = 0; u < (F.term[c][d].merged ? 1 : 2); ++u) {
+        const FzOp& o = u ? F.term[c][d].b : F.term[c][d].a;
+        if (d == 1 ? !(c == 1 ? c2p(o, true, false) : p2c(o, true)) : !per(o, d == 0 ? dx : dz)) return false;
+      }
+  return per(F.pres[0], dx) && c2p(F.pres[1], true, false) && per(F.pres[2], dz);
+}
+
 // Momentum right-hand sides, fractional step, mass-flux mean and advance of the substep in four
 // launches (wall planes, fused momentum, mean, advance) instead of the ~50 of the operator path.
 // Returns false (nothing launched) when the configuration needs the operator path.
@@ -1373,7 +1466,9 @@ bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz,
   F.pres[2] = b.op(2, D1C2P, bz_pr, true);
   F.fpres[0] = any; F.fpres[1] = fympr; F.fpres[2] = any;
   if (!b.ok) return false;
-  if (H->idriven == 1) {
+  F.adv = defer_update ? (advances_x<T>(H) ? 7 : 6) : 0;
+  const bool march = fz_march_form(H, F);
+  if (H->idriven == 1 && !march) {
     F.wy = H->wy;
     F.part = H->fz_part;
   }
@@ -1389,7 +1484,40 @@ bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz,
           bufs(H->fb_visc2, H->fb_comb), launch_fz_wall_visc<T>(F, A(H->fb_visc2), A(H->fb_comb), fconv2, st));
     H->launches++;
   }
-  {
+  const double* bulk = H->idriven == 1 ? H->scal + 0 : nullptr;
+  if (march) {
+    if (!H->periodic_y) {
+      // the y component's wall rows, beside the march: fb_visc2 stands for them in the schedule, as the
+      // march writes the other rows of the same arrays
+      PROFD(H, 3, (double)sizeof(T) * 40.0 * nc0 * nc2,
+            bufs(H->qx, H->qy, H->qz, H->pres, TH ? H->gx : nullptr, TH ? H->gy : nullptr, TH ? H->gz : nullptr,
+                 TH ? H->mVisc : nullptr, H->fb_comb, H->fb_conv2, H->fb_qx, H->fb_qz, H->fb_qy,
+                 TH ? H->fb_m : nullptr),
+            bufs(H->fb_visc2), launch_fz_wall_rows<T>(F, st));
+      H->launches++;
+    }
+    FzMarch<T> M{};
+    M.n0 = nc0; M.nc1 = nc1; M.np1 = np1; M.n2 = nc2;
+    const T* in[8] = {F.qx, F.qy, F.qz, F.p, F.gx, F.gy, F.gz, F.mu};
+    for (int q = 0; q < 8; ++q) M.a[q] = in[q];
+    M.bqx = F.fyqx; M.bqz = F.fyqz; M.bg = F.fz; M.bmu = F.fm;
+    M.wp = H->fz_w; M.wc = H->fz_w + np1;
+    M.dxi = 1.0 / H->h[0]; M.dzi = 1.0 / H->h[2];
+    M.rre = F.rre; M.dt = F.dt; M.gam = F.gam; M.zeta = F.zeta; M.alpha = F.alpha;
+    for (int c = 0; c < 3; ++c) { M.out[c] = F.m[c]; M.m0[c] = F.m0[c]; }
+    M.adv = F.adv;
+    if (H->idriven == 1) {
+      M.wy = H->wy; M.part = H->fz_part; M.count = H->fz_count; M.bulk = H->scal + 0; M.vol = H->vol;
+    }
+    // q (3), p [, g (3), mu] and the histories read, histories and increments written
+    PROFD(H, 4, nf * ((TH ? 8.0 : 4.0) + 9.0),
+          bufs(H->qx, H->qy, H->qz, H->pres, TH ? H->gx : nullptr, TH ? H->gy : nullptr, TH ? H->gz : nullptr,
+               TH ? H->mVisc : nullptr, H->fb_qx, H->fb_qz, TH ? H->fb_m : nullptr, TH ? H->fb_zero : nullptr),
+          bufs(H->mx, H->my, H->mz, H->mx0, H->my0, H->mz0, M.part, M.part ? H->scal : nullptr,
+               M.part ? H->fz_count : nullptr),
+          launch_fz_march<T>(M, TH, H->periodic_y, st));
+    H->launches++;
+  } else {
     // one pass per component: rhs0 read and written, rhs written, and a third of the shared inputs
     // q (3), p [+ g (3), mu] (the three components together read each input once); the three run
     // concurrently on the dataflow lanes, x and z also beside the wall-row kernel (only the y
@@ -1404,19 +1532,17 @@ bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz,
             bufs(mo[c], m0[c], c == 0 && F.part ? H->fz_part : nullptr), launch_fz_momentum<T>(F, c, st));
       H->launches++;
     }
-  }
-  const double* bulk = nullptr;
-  if (H->idriven == 1) {
-    // the mass-flux mean from the x pass's per-CTA sums
-    const int nblk = fz_momentum_x_blocks(nc0, nc1, nc2);
-    PROFD(H, 3, 8.0 * nblk, bufs(H->fz_part), bufs(H->scal),
-          launch_fz_finalize_mean(H->fz_part, nblk, H->scal + 0, H->vol, st));
-    bulk = H->scal + 0;
-    H->launches++;
+    if (bulk) {
+      // the mass-flux mean from the x pass's per-CTA sums
+      const int nblk = fz_momentum_x_blocks(nc0, nc1, nc2);
+      PROFD(H, 3, 8.0 * nblk, bufs(H->fz_part), bufs(H->scal),
+            launch_fz_finalize_mean(H->fz_part, nblk, H->scal + 0, H->vol, st));
+      H->launches++;
+    }
   }
   if (defer_update) return true;  // the advance is folded into fused_update_div and fused_project
   const int w0 = B[1][V_QY][0] == BC_DIRICHLET, w1 = B[1][V_QY][1] == BC_DIRICHLET;
-  PROFD(H, 3, nf * 9.0, bufs(H->mx, H->my, H->mz, bulk), bufs(ux, uy, uz),
+  PROFD(H, 3, nf * 9.0, bufs(H->mx, H->my, H->mz, bulk, H->fb_visc2), bufs(ux, uy, uz),
         launch_fz_update<T>(A(ux), A(uy), A(uz), A(H->mx), A(H->my), A(H->mz), bulk, nc0, nc1, np1, nc2, w0,
                             H->fbcy[V_QY][0], w1, H->fbcy[V_QY][1], st));
   H->launches++;
@@ -1426,15 +1552,15 @@ bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz,
 // The Poisson right-hand side with the momentum advance folded in (FzUpdateDiv); launch false:
 // only whether it can run.
 template <typename T>
-bool fused_update_div(chs_handle* H, int isub, double* ux, double* uy, double* uz, int w0, int w1, bool launch) {
+bool fused_update_div(chs_handle* H, int isub, double* ux, int w0, int w1, bool launch) {
   if (!H->kfuse || H->iacc != ACC_CD2 || !H->fz_rows) return false;
   auto A = [](double* p) { return reinterpret_cast<T*>(p); };
   const auto& B = H->ibc;
   FzBuild b{H};
   FzUpdateDiv<T> F{};
   F.n0 = H->nc[0]; F.nc1 = H->nc[1]; F.np1 = H->np[1]; F.n2 = H->nc[2];
-  F.ux = A(ux); F.uy = A(uy); F.uz = A(uz);
-  F.mx = A(H->mx); F.my = A(H->my); F.mz = A(H->mz);
+  F.ux = A(H->mx); F.uy = A(H->my); F.uz = A(H->mz);
+  if (!advances_x<T>(H)) { F.ux = A(ux); F.mx = A(H->mx); }
   F.bulk = H->idriven == 1 ? H->scal + 0 : nullptr;
   F.s0 = w0; F.s1 = w1;
   F.v0 = H->fbcy[V_QY][0]; F.v1 = H->fbcy[V_QY][1];
@@ -1449,7 +1575,7 @@ bool fused_update_div(chs_handle* H, int isub, double* ux, double* uy, double* u
   if (!b.ok || H->periodic_y) return false;
   if (!launch) return true;
   const double nf = (double)sizeof(T) * H->n_ccc;
-  PROFD(H, 4, nf * 7.0, bufs(ux, uy, uz, H->mx, H->my, H->mz, F.bulk), bufs(H->pcor),
+  PROFD(H, 4, nf * (F.mx ? 5.0 : 4.0), bufs(F.mx ? ux : nullptr, H->mx, H->my, H->mz, H->fb_visc2, F.bulk), bufs(H->pcor),
         launch_fz_update_div<T>(F, st));
   H->launches++;
   return true;
@@ -1566,14 +1692,14 @@ bool fused_project(chs_handle* H, int isub, double* ux, double* uy, double* uz, 
   F.s0 = w0; F.s1 = w1;
   F.v0 = H->fbcy[V_QY][0]; F.v1 = H->fbcy[V_QY][1];
   F.rows = H->fz_rows;
-  F.upd = upd ? 1 : 0;
+  F.upd = upd ? (advances_x<T>(H) ? 1 : 2) : 0;
   F.mx = A(H->mx); F.my = A(H->my); F.mz = A(H->mz);
   F.bulk = H->idriven == 1 ? H->scal + 0 : nullptr;
   if (!launch) return true;
   const double nf = (double)sizeof(T) * H->n_ccc;
-  PROFD(H, 3, nf * (TH ? 13.0 : 9.0) + (upd ? 3.0 * nf : 0.0),
+  PROFD(H, 3, nf * (TH ? 13.0 : 9.0),
         bufs(H->pcor, H->fb_pr, TH ? H->dDens : nullptr, TH ? H->fb_d : nullptr, upd ? H->mx : nullptr,
-             upd ? H->my : nullptr, upd ? H->mz : nullptr, upd ? F.bulk : nullptr),
+             upd ? H->my : nullptr, upd ? H->mz : nullptr, upd ? F.bulk : nullptr, upd ? H->fb_visc2 : nullptr),
         bufs(H->pres, ux, uy, uz, TH ? H->qx : nullptr, TH ? H->qy : nullptr, TH ? H->qz : nullptr),
         launch_fz_project<T>(F, st));
   H->launches++;
@@ -1613,7 +1739,7 @@ void substep_body_t(chs_handle* H, int isub, int parts) {
   const int w0 = B[1][V_QY][0] == BC_DIRICHLET, w1 = B[1][V_QY][1] == BC_DIRICHLET;
   // fused path: the momentum advance u += m - bulk is not stored by itself but formed where the
   // Poisson right-hand side and the projection read u (both fused kernels must be available)
-  const bool defer = fused_update_div<T>(H, isub, ux, uy, uz, w0, w1, false) &&
+  const bool defer = fused_update_div<T>(H, isub, ux, w0, w1, false) &&
                      fused_project<T>(H, isub, ux, uy, uz, w0, w1, true, false);
   const bool mom_fused = fused_momentum<T>(H, isub, ux, uy, uz, defer);
   const bool upd = defer && mom_fused;
@@ -1778,7 +1904,7 @@ void substep_body_t(chs_handle* H, int isub, int parts) {
   // Update_thermal_properties has already set rho_m1 = rho, so the term is zero and left out.
   const double coeff = 1.0 / (H->tAlpha[isub] * H->sigma2p * H->dt);
   if (upd) {
-    fused_update_div<T>(H, isub, ux, uy, uz, w0, w1, true);
+    fused_update_div<T>(H, isub, ux, w0, w1, true);
   } else {
     std::vector<OpTerm<T>> t = {term<T>(0, D1P2C, bx_qx, any, src(A(ux)), s_pcc, coeff, 0),
                                 term<T>(1, D1P2C, by_qy, nullptr, src(A(uy)), s_cpc, coeff, 0),
