@@ -29,6 +29,7 @@ constexpr int kRows = kTY + 2;   // rows of a set: j0 - 1 .. j0 + kTY
 constexpr int kXS = 36;          // columns of a set: i0 - 2 .. i0 + 33
 constexpr int kSets = 3;
 constexpr int kThreads = (kTY + 2) * 32;
+constexpr int kWall = 2 * 4 * kXS;  // wall planes' rows in a set: below, above of qx, qz, momentum, mu
 
 // two values (16 or 8 bytes) from global to shared memory
 template <typename T>
@@ -41,6 +42,7 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 enum { QX, QY, QZ, PR, GX, GY, GZ, MU };
+enum { WQX, WQZ, WG, WMU };
 
 template <typename T>
 struct Exchange {
@@ -54,65 +56,74 @@ struct Exchange {
 };
 
 template <typename T, bool TH>
-constexpr size_t march_smem() {
-  return (size_t)kSets * (TH ? 8 : 4) * kRows * kXS * sizeof(T) + sizeof(Exchange<T>);
-}
+struct MarchSize {
+  static constexpr int fields = TH ? 8 : 4;
+  static constexpr int pairs = fields * kRows * (kXS / 2);             // pair copies of a set
+  static constexpr int copies = (pairs + kThreads - 1) / kThreads;     // per thread
+  static constexpr int set = fields * kRows * kXS + kWall;             // values of a set
+  static constexpr size_t smem = (size_t)kSets * set * sizeof(T) + (size_t)copies * kThreads * 8 + sizeof(Exchange<T>);
+};
 
 template <typename T, bool TH, bool PY>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
     fz_march_kernel(const __grid_constant__ FzMarch<T> f) {
-  constexpr int NF = TH ? 8 : 4;
-  constexpr int kSet = NF * kRows * kXS;             // values of a set
-  constexpr int kPairs = NF * kRows * (kXS / 2);     // pair copies of a set
-  constexpr int kCopies = (kPairs + kThreads - 1) / kThreads;
+  using Sz = MarchSize<T, TH>;
+  constexpr int kSet = Sz::set, kCopies = Sz::copies, kData = Sz::fields * kRows * kXS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
-  Exchange<T>& ex = *reinterpret_cast<Exchange<T>*>(ring + kSets * kSet);
+  const T** from = reinterpret_cast<const T**>(ring + kSets * kSet);  // [copies][threads]
+  Exchange<T>& ex = *reinterpret_cast<Exchange<T>*>(from + kCopies * kThreads);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int n0 = f.n0, ny = f.nc1, np1 = f.np1, n2 = f.n2, nl = n0 * n2;
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * kTY;
   const int k0 = blockIdx.z * f.chunk, k1 = min(k0 + f.chunk, n2);
   auto wrapk = [&](int k) { return k < 0 ? k + n2 : (k >= n2 ? k - n2 : k); };
 
-  // ---- this thread's share of a set: the offset of every pair within its array's plane
-  int goff[kCopies];
+  // ---- this thread's share of a set: copy u is pair threadIdx.x + u * kThreads of the set, from plane 0's
+  // address in `from` (its own slots only) and, by the two bits of `kinds`, the plane offset of a
+  // cell-centred array (0), of y points (1; ny + 1 rows with walls) or of z points (2; plane k + 1)
+  unsigned kinds = 0;
 #pragma unroll
   for (int u = 0; u < kCopies; ++u) {
     const int e = threadIdx.x + u * kThreads;
+    if (e >= Sz::pairs) continue;
     const int fld = e / (kRows * (kXS / 2)), r = e / (kXS / 2) % kRows, c = e % (kXS / 2) * 2;
-    const bool pts = fld == QY || fld == GY;  // y points (ny + 1 rows with walls), else y cells
-    const int rows = pts ? np1 : ny;
+    const bool pts = fld == QY || fld == GY;
     int i = i0 - 2 + c, j = j0 - 1 + r;
     i = ((i % n0) + n0) % n0;
-    j = PY ? ((j % ny) + ny) % ny : min(max(j, 0), rows - 1);
-    goff[u] = j * n0 + i;
+    j = PY ? ((j % ny) + ny) % ny : min(max(j, 0), (pts ? np1 : ny) - 1);
+    from[u * kThreads + threadIdx.x] = f.a[fld] + (j * n0 + i);
+    kinds |= (pts ? 1u : (fld == QZ || fld == GZ) ? 2u : 0u) << (2 * u);
   }
-  // plane k of every array, plane k + 1 of qz and gz (z points: the cell's two z faces)
+  // wall rows: the pair this thread copies (threads 0 .. 143; null: none)
+  const T* wall_from = nullptr;
+  if (!PY && threadIdx.x < kWall / 2) {
+    const int sd = threadIdx.x / (kWall / 4), q = threadIdx.x / (kXS / 2) % 4, c = threadIdx.x % (kXS / 2) * 2;
+    const T* b = q == WQX ? f.bqx : (q == WQZ ? f.bqz : (q == WG ? f.bg : f.bmu));
+    const bool has = sd == 0 ? j0 == 0 : j0 + kTY >= ny;
+    int i = i0 - 2 + c;
+    i = ((i % n0) + n0) % n0;
+    if (has && (TH || q < WG)) wall_from = b + sd * nl + i;
+  }
   auto load_set = [&](int k, T* set, bool z_only) {
     const int kw = wrapk(k), kz = wrapk(k + 1);
+    const int off_c = kw * ny * n0, off_y = kw * np1 * n0, off_z = kz * ny * n0;
 #pragma unroll
     for (int u = 0; u < kCopies; ++u) {
       const int e = threadIdx.x + u * kThreads;
-      if (e < kPairs) {
-        const int fld = e / (kRows * (kXS / 2)), rc = e % (kRows * (kXS / 2));
-        const bool z = fld == QZ || fld == GZ;
-        if (z || !z_only) {
-          const int plane = ((fld == QY || fld == GY) ? np1 : ny) * n0;
-          copy_pair(set + fld * (kRows * kXS) + rc * 2, f.a[fld] + ((z ? kz : kw) * plane + goff[u]));
-        }
+      if (e < Sz::pairs) {
+        const unsigned kind = kinds >> (2 * u) & 3u;
+        if (kind == 2u || !z_only)
+          copy_pair(set + 2 * e, from[u * kThreads + threadIdx.x] + (kind == 0u ? off_c : (kind == 1u ? off_y : off_z)));
       }
     }
+    if (wall_from && !z_only) copy_pair(set + kData + 2 * threadIdx.x, wall_from + kw * n0);
   };
 
   const T half = T(0.5), third = T(1.0 / 3.0), dxi = T(f.dxi), dzi = T(f.dzi), rre = T(f.rre);
   // y weights of row j (cells) and edge j (points)
   auto wcell = [&](int j) { return T(f.wc[PY ? (j + ny) % ny : min(max(j, 0), ny - 1)]); };
   auto wedge = [&](int j) { return T(f.wp[PY ? (j + ny) % ny : min(max(j, 0), np1 - 1)]); };
-  // column of the arrays that set column c holds
-  auto col = [&](int c) {
-    int i = i0 - 2 + c;
-    return ((i % n0) + n0) % n0;
-  };
 #define V(S, F, R, C) (S)[((F) * kRows + (R)) * kXS + (C)]
 
   // ---- the stresses.  A: the set of plane k (qz, gz: k + 1), B: of k - 1 (qz, gz: k); set row r, column c
@@ -138,30 +149,30 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
     return rre * v - m * q;
   };
   // rows r and r - 1 of a y-cell array at edge r; beyond a wall (side 1 below, 2 above) the value that
-  // puts the wall's in the middle
-  auto ypair = [&](const T* S, int fld, int r, int c, const T* wall, int k, int side, T& hi, T& lo) {
+  // puts the wall's (row q of the wall rows of set Wl) in the middle
+  auto ypair = [&](const T* S, int fld, int r, int c, const T* Wl, int q, int side, T& hi, T& lo) {
     hi = V(S, fld, r, c);
     lo = V(S, fld, r - 1, c);
     if (!PY && side) {
-      const int at = col(c) + n0 * wrapk(k);
-      if (side == 1) lo = T(2) * __ldg(wall + at) - hi;
-      else hi = T(2) * __ldg(wall + nl + at) - lo;
+      const T b = Wl[kData + ((side - 1) * 4 + q) * kXS + c];
+      if (side == 1) lo = T(2) * b - hi;
+      else hi = T(2) * b - lo;
     }
   };
   // xy edge: the x component's stress e0 and the y component's e1
-  auto edge_xy = [&](const T* A, int r, int c, T wp, int k, int side, T& e0, T& e1) {
+  auto edge_xy = [&](const T* A, int r, int c, T wp, int side, T& e0, T& e1) {
     T qh, ql;
-    ypair(A, QX, r, c, f.bqx, k, side, qh, ql);
+    ypair(A, QX, r, c, A, WQX, side, qh, ql);
     const T qyr = V(A, QY, r, c), qyl = V(A, QY, r, c - 1);
     const T qxi = half * (qh + ql), qyi = half * (qyr + qyl);
     T v = wp * (qh - ql) + dxi * (qyr - qyl);
     T m0 = qyi, m1 = qxi;
     if (TH) {
       T mh, ml, nh, nlo, gh, gl;
-      ypair(A, MU, r, c, f.bmu, k, side, mh, ml);
-      ypair(A, MU, r, c - 1, f.bmu, k, side, nh, nlo);
+      ypair(A, MU, r, c, A, WMU, side, mh, ml);
+      ypair(A, MU, r, c - 1, A, WMU, side, nh, nlo);
       v *= half * (half * (mh + ml) + half * (nh + nlo));
-      ypair(A, GX, r, c, f.bg, k, side, gh, gl);
+      ypair(A, GX, r, c, A, WG, side, gh, gl);
       m0 = half * (V(A, GY, r, c) + V(A, GY, r, c - 1));
       m1 = half * (gh + gl);
     }
@@ -185,19 +196,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
     e2 = v - m2 * qzi;
   };
   // yz edge: of the y component (e1) and the z component (e2)
-  auto edge_yz = [&](const T* A, const T* B, int r, int c, T wp, int k, int side, T& e1, T& e2) {
+  auto edge_yz = [&](const T* A, const T* B, int r, int c, T wp, int side, T& e1, T& e2) {
     T zh, zl;
-    ypair(B, QZ, r, c, f.bqz, k, side, zh, zl);
+    ypair(B, QZ, r, c, A, WQZ, side, zh, zl);
     const T ya = V(A, QY, r, c), yb = V(B, QY, r, c);
     const T qyi = half * (ya + yb), qzi = half * (zh + zl);
     T v = wp * (zh - zl) + dzi * (ya - yb);
     T m1 = qzi, m2 = qyi;
     if (TH) {
       T mh, ml, nh, nlo, gh, gl;
-      ypair(A, MU, r, c, f.bmu, k, side, mh, ml);
-      ypair(B, MU, r, c, f.bmu, k - 1, side, nh, nlo);
+      ypair(A, MU, r, c, A, WMU, side, mh, ml);
+      ypair(B, MU, r, c, B, WMU, side, nh, nlo);
       v *= half * (half * (mh + ml) + half * (nh + nlo));
-      ypair(B, GZ, r, c, f.bg, k, side, gh, gl);
+      ypair(B, GZ, r, c, A, WG, side, gh, gl);
       m1 = half * (gh + gl);
       m2 = half * (V(A, GY, r, c) + V(B, GY, r, c));
     }
@@ -213,8 +224,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
   const int i = i0 + lane, j = j0 + w, r = w + 1, c = lane + 2;
   const bool valid = outw && i < n0 && j < ny;
   const bool yval = valid && (PY || j > 0);  // wall rows of the y component: fz_wall_rows_kernel
-  const T wc = wcell(j), wp = wedge(j);
-  const int side = side_of(j);
+  // the row whose weights the warp's stresses take: its own, the tile's outer rows (normal stress below,
+  // edges above), or one row per eight lanes
+  const int jh = j0 + (lane & 7);
+  const T wc = wcell(outw ? j : (w == kTY ? j0 - 1 : jh)), wp = wedge(outw ? j : (w == kTY ? j0 + kTY : jh));
+  const int side = side_of(outw ? j : (w == kTY ? j0 + kTY : jh));
   const T dt = T(f.dt), gam = T(f.gam), zeta = T(f.zeta), alpha = T(f.alpha);
   T zz = T(0), xz0 = T(0), yz1 = T(0);    // of the previous plane
   T fx = T(0), fy = T(0), ax = T(0), ay = T(0), ux = T(0), uy = T(0);  // pending x and y components
@@ -247,12 +261,12 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
       if (k < k1) nzz = normal(A, B, r, c, wc, 2);
       if (k >= k0) {
         edge_xz(A, B, r, c, nxz0, xz2);
-        edge_yz(A, B, r, c, wp, k, side, nyz1, yz2);
+        edge_yz(A, B, r, c, wp, side, nyz1, yz2);
       }
       if (inner) {
         xx = normal(A, B, r, c, wc, 0);
         yy = normal(A, B, r, c, wc, 1);
-        edge_xy(A, r, c, wp, k, side, xy0, xy1);
+        edge_xy(A, r, c, wp, side, xy0, xy1);
         ex.xx[w][lane + 1] = xx;
         ex.xy1[w][lane] = xy1;
         ex.xz2[w][lane] = xz2;
@@ -264,20 +278,18 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
       T t0, t1;
       if (w == kTY) {
         // the rows beyond the tile
-        ex.yy[0][lane] = normal(A, B, 0, c, wcell(j0 - 1), 1);
-        const int jt = j0 + kTY, st = side_of(jt);
-        const T wt = wedge(jt);
-        edge_xy(A, kTY + 1, c, wt, k, st, t0, t1);
+        ex.yy[0][lane] = normal(A, B, 0, c, wc, 1);
+        edge_xy(A, kTY + 1, c, wp, side, t0, t1);
         ex.xy0[kTY][lane] = t0;
-        edge_yz(A, B, kTY + 1, c, wt, k, st, t0, t1);
+        edge_yz(A, B, kTY + 1, c, wp, side, t0, t1);
         ex.yz2[kTY][lane] = t1;
       } else {
         // the columns beyond the tile: 8 lanes per stress, one row each
-        const int q = lane & 7, jq = j0 + q;
+        const int q = lane & 7;
         if (lane < 8) {
-          ex.xx[q][0] = normal(A, B, q + 1, 1, wcell(jq), 0);
+          ex.xx[q][0] = normal(A, B, q + 1, 1, wc, 0);
         } else if (lane < 16) {
-          edge_xy(A, q + 1, 34, wedge(jq), k, side_of(jq), t0, t1);
+          edge_xy(A, q + 1, 34, wp, side, t0, t1);
           ex.xy1[q][32] = t1;
         } else if (lane < 24) {
           edge_xz(A, B, q + 1, 34, t0, t1);
@@ -367,8 +379,8 @@ dim3 march_grid(int n0, int ny, int n2, int& chunk) {
   // planes of a run, each run paying two planes more than it owns
   int occ = 1;
   cudaFuncSetAttribute(fz_march_kernel<T, TH, PY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)march_smem<T, TH>());
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fz_march_kernel<T, TH, PY>, kThreads, march_smem<T, TH>());
+                       (int)MarchSize<T, TH>::smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fz_march_kernel<T, TH, PY>, kThreads, MarchSize<T, TH>::smem);
   const int64_t tiles = (int64_t)((n0 + 31) / 32) * ((ny + kTY - 1) / kTY), slots = 148 * (int64_t)std::max(occ, 1);
   double best = 1e300;
   chunk = n2;
@@ -386,7 +398,7 @@ dim3 march_grid(int n0, int ny, int n2, int& chunk) {
 template <typename T, bool TH, bool PY>
 void launch_march_t(FzMarch<T> f, cudaStream_t st) {
   const dim3 grid = march_grid<T, TH, PY>(f.n0, f.nc1, f.n2, f.chunk);
-  fz_march_kernel<T, TH, PY><<<grid, kThreads, march_smem<T, TH>(), st>>>(f);
+  fz_march_kernel<T, TH, PY><<<grid, kThreads, MarchSize<T, TH>::smem, st>>>(f);
 }
 
 }  // namespace
