@@ -61,7 +61,9 @@ void launch_line_chunk(int d, const OpPlan& P, const LineIOT<T>& io, const doubl
 
 // nondimensional property table on the device, sorted by T (FP64 columns)
 struct ThermoTab {
-  const double *t, *h, *d, *m, *k, *rhoh;
+  const double* t;
+  // by row, ' the slope to the next one: (rho*h, h) (h', 0) and (h, rho) (rho', mu) (mu', kappa) (kappa', T) (T', 0)
+  const double2 *rh, *hp;
   int n;
   double dhmin, dhmax;
   // bracket index of the rho*h (0) and h (1) columns: for each of ix_nb uniform bins over

@@ -378,10 +378,7 @@ __global__ void __launch_bounds__(128, 6) mlp_props_kernel(
         const double f = (y[0] - ck.t0) / ck.dt_tab;
         if (f >= 0.0 && f <= (double)(tb.n - 1)) hint = (int)f;
       } else if (y[0] >= __ldg(tb.t) && y[0] <= __ldg(tb.t + tb.n - 1)) {
-        int i1, i2;
-        double w1;
-        tab_bracket(tb.t, tb.n, y[0], i1, i2, w1);
-        hint = i1;
+        hint = tab_row(tb.t, tb.n, y[0]);
       }
       bool hit = false;
       const CellProps p = props_from_dh(tb, rh, hint, ck.win, &hit);

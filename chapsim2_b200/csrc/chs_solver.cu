@@ -2141,11 +2141,25 @@ void thermo_init(chs_handle* H, const chs_thermo* c) {
       throw std::invalid_argument("rho*h and h must increase with T for the rho*h lookup");
   }
   if (!(c->t_ini >= c->t[0] && c->t_ini <= c->t[n - 1])) throw std::invalid_argument("t_ini outside the table");
-  double* cols = H->dalloc<double>((size_t)6 * n);
-  const double* srcs[6] = {c->t, c->h, c->d, c->m, c->k, rhoh.data()};
-  for (int j = 0; j < 6; ++j)
-    CK(cudaMemcpyAsync(cols + (size_t)j * n, srcs[j], n * sizeof(double), cudaMemcpyHostToDevice, H->st));
-  H->tab = ThermoTab{cols, cols + n, cols + 2 * n, cols + 3 * n, cols + 4 * n, cols + 5 * n, n,
+  double* tcol = H->dalloc<double>(n);
+  CK(cudaMemcpyAsync(tcol, c->t, n * sizeof(double), cudaMemcpyHostToDevice, H->st));
+  std::vector<double2> pairs(7 * (size_t)n, make_double2(0.0, 0.0));
+  for (int i = 0; i < n; ++i) {
+    // the last row starts no interval
+    auto slope = [&](const double* y, const double* x) { return i + 1 < n ? (y[i + 1] - y[i]) / (x[i + 1] - x[i]) : 0.0; };
+    pairs[2 * i] = make_double2(rhoh[i], c->h[i]);
+    pairs[2 * i + 1].x = slope(c->h, rhoh.data());
+    double2* r = pairs.data() + 2 * (size_t)n + 5 * (size_t)i;
+    r[0] = make_double2(c->h[i], c->d[i]);
+    r[1] = make_double2(slope(c->d, c->h), c->m[i]);
+    r[2] = make_double2(slope(c->m, c->h), c->k[i]);
+    r[3] = make_double2(slope(c->k, c->h), c->t[i]);
+    r[4].x = slope(c->t, c->h);
+  }
+  double2* pd = H->dalloc<double2>(pairs.size());
+  CK(cudaMemcpyAsync(pd, pairs.data(), pairs.size() * sizeof(double2), cudaMemcpyHostToDevice, H->st));
+  CK(cudaStreamSynchronize(H->st));  // the pairs are a local array
+  H->tab = ThermoTab{tcol, pd, pd + 2 * n, n,
                      *std::min_element(rhoh.begin(), rhoh.end()), *std::max_element(rhoh.begin(), rhoh.end())};
   {
     // bracket index of the strictly increasing rho*h and h columns (2n bins each).  For x fixed,
