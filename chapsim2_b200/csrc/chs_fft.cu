@@ -1,7 +1,6 @@
 // FFTs of the Poisson solvers in at most three stages held in registers.
 //
-// A length n = 2^a 3^b up to 729 factors into at most three radices of 2, 3, 4, 6, 8, 9 (fft_stages in
-// chs_plan.cpp), the largest in the middle.  The first Stockham stage takes its inputs from global memory and
+// A length n = 2^a 3^b up to 729 factors into at most three radices of 2, 3, 4, 6, 8, 9 (fft_stages), the largest in the middle.  The first Stockham stage takes its inputs from global memory and
 // the last stores its results there, so a line passes through shared memory once per stage boundary (twice
 // at most); the middle stage works in place, one butterfly per thread between two barriers.  The tile
 // has the lines side by side (z and y lines, whose 16 or 32 neighbouring columns are one 256-byte
@@ -13,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <stdexcept>
 
 #include "chs_kernels.cuh"
@@ -210,8 +210,9 @@ __global__ void __launch_bounds__(512, 2) cfft_lines_kernel(const __grid_constan
   C* tw = reinterpret_cast<C*>(fft_smem);
   C* tile = tw + fp.n;
   const int lines = 1 << lsh;
+  grid_dep_launch();
   copy_twiddles(fp, tw);
-  if (fp.rst == 1) __syncthreads();
+  grid_dep_wait();
   // blockDim is a multiple of `lines`: a thread keeps its line
   const int l = threadIdx.x & (lines - 1), g = (blockIdx.x << lsh) + l;
   const bool ok = g < nlines;
@@ -237,6 +238,7 @@ __global__ void __launch_bounds__(512, 2) rfft_rows_kernel(const __grid_constant
   C* tw = reinterpret_cast<C*>(fft_smem);
   C* tile = tw + fp.n;
   const int n = fp.n, nh = n / 2 + 1, ls = pad9(n) + 1, pair0 = blockIdx.x * pairs;
+  grid_dep_launch();
   copy_twiddles(fp, tw);
   auto split = [&](int t, int nb, int& ln, int& j) {
     ln = div_small(t, nb, 1.0f / (float)nb);
@@ -287,8 +289,9 @@ __global__ void __launch_bounds__(512, 2) irfft_rows_kernel(const __grid_constan
   C* tw = reinterpret_cast<C*>(fft_smem);
   C* tile = tw + fp.n;
   const int n = fp.n, nh = n / 2 + 1, ls = pad9(n) + 1, pair0 = blockIdx.x * pairs;
+  grid_dep_launch();
   copy_twiddles(fp, tw);
-  if (fp.rst == 1) __syncthreads();
+  grid_dep_wait();
   const S sc = (S)scale;
   auto split = [&](int t, int nb, int& ln, int& j) {
     ln = div_small(t, nb, 1.0f / (float)nb);
@@ -340,6 +343,32 @@ void allow_smem(K kernel, size_t shm) {
 
 }  // namespace
 
+void fft_stages(FftPlan& fp) {
+  // fewest stages, then the smallest sum of radices; the largest in the middle of three, else last
+  static const int rad[6] = {2, 3, 4, 6, 8, 9};
+  fp.rst = 0;
+  int best = 1 << 30;
+  auto take = [&](std::initializer_list<int> r) {
+    int n = 1, sum = 0, k = 0;
+    for (int x : r) { n *= x; sum += x; }
+    if (n != fp.n || (fp.rst && ((int)r.size() > fp.rst || ((int)r.size() == fp.rst && sum >= best)))) return;
+    fp.rst = (int)r.size();
+    best = sum;
+    for (int x : r) fp.rrad[k++] = x;
+    std::sort(fp.rrad, fp.rrad + k);
+    if (k == 3) std::swap(fp.rrad[1], fp.rrad[2]);
+  };
+  for (int a : rad) {
+    take({a});
+    for (int b : rad) {
+      if (b < a) continue;
+      take({a, b});
+      for (int c : rad)
+        if (c >= b) take({a, b, c});
+    }
+  }
+}
+
 template <typename R, typename C>
 void launch_rfft_rows(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream_t st) {
   const int npairs = (nrows + 1) / 2, pairs = row_pairs(fp, npairs), n = fp.n;
@@ -349,16 +378,16 @@ void launch_rfft_rows(const FftPlan& fp, const R* in, C* out, int nrows, cudaStr
                                                                                                   pairs);
 }
 template <typename R, typename C>
-void launch_irfft_rows(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st) {
+void launch_irfft_rows(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st, bool chained) {
   const int npairs = (nrows + 1) / 2, pairs = row_pairs(fp, npairs), n = fp.n;
   const size_t shm = ((size_t)n + (size_t)pairs * (n + n / 8 + 1)) * sizeof(C);
   allow_smem(irfft_rows_kernel<R, C>, shm);
-  irfft_rows_kernel<R, C><<<(npairs + pairs - 1) / pairs, fft_threads(fp, pairs, false), shm, st>>>(
-      fp, in, out, nrows, scale, pairs);
+  launch_chained(irfft_rows_kernel<R, C>, dim3((npairs + pairs - 1) / pairs), dim3(fft_threads(fp, pairs, false)), shm,
+                 st, chained, fp, in, out, nrows, scale, pairs);
 }
 template <typename C>
 void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstride, int64_t stride, int sign,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool chained) {
   const int64_t nlines = (int64_t)na * nb;
   if (nlines > 0x3fffffff) throw std::runtime_error("FFT: too many lines");
   // 256-byte segments, narrower while the tile exceeds 64 KB or the CTA 512 threads
@@ -366,16 +395,20 @@ void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstri
   while (lsh > 2 && (((size_t)fp.n << lsh) * sizeof(C) > 64 * 1024 || fft_threads(fp, 1 << lsh, false) > 512)) --lsh;
   const size_t shm = ((size_t)fp.n + ((size_t)fp.n << lsh)) * sizeof(C);
   allow_smem(cfft_lines_kernel<C>, shm);
-  cfft_lines_kernel<C><<<(unsigned)((nlines + (1 << lsh) - 1) >> lsh), fft_threads(fp, 1 << lsh, false), shm, st>>>(
-      fp, data, na, (int)nlines, bstride, stride, sign, lsh);
+  launch_chained(cfft_lines_kernel<C>, dim3((unsigned)((nlines + (1 << lsh) - 1) >> lsh)),
+                 dim3(fft_threads(fp, 1 << lsh, false)), shm, st, chained, fp, data, na, (int)nlines, bstride, stride, sign,
+                 lsh);
 }
 template void launch_rfft_rows<double, double2>(const FftPlan&, const double*, double2*, int, cudaStream_t);
 template void launch_rfft_rows<float, double2>(const FftPlan&, const float*, double2*, int, cudaStream_t);
 template void launch_rfft_rows<float, float2>(const FftPlan&, const float*, float2*, int, cudaStream_t);
-template void launch_irfft_rows<double, double2>(const FftPlan&, const double2*, double*, int, double, cudaStream_t);
-template void launch_irfft_rows<float, double2>(const FftPlan&, const double2*, float*, int, double, cudaStream_t);
-template void launch_irfft_rows<float, float2>(const FftPlan&, const float2*, float*, int, double, cudaStream_t);
-template void launch_cfft_lines<double2>(const FftPlan&, double2*, int, int, int64_t, int64_t, int, cudaStream_t);
-template void launch_cfft_lines<float2>(const FftPlan&, float2*, int, int, int64_t, int64_t, int, cudaStream_t);
+template void launch_irfft_rows<double, double2>(const FftPlan&, const double2*, double*, int, double, cudaStream_t,
+                                                 bool);
+template void launch_irfft_rows<float, double2>(const FftPlan&, const double2*, float*, int, double, cudaStream_t,
+                                                 bool);
+template void launch_irfft_rows<float, float2>(const FftPlan&, const float2*, float*, int, double, cudaStream_t,
+                                                 bool);
+template void launch_cfft_lines<double2>(const FftPlan&, double2*, int, int, int64_t, int64_t, int, cudaStream_t, bool);
+template void launch_cfft_lines<float2>(const FftPlan&, float2*, int, int, int64_t, int64_t, int, cudaStream_t, bool);
 
 }  // namespace chs

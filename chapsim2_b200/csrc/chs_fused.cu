@@ -588,6 +588,8 @@ __global__ void __launch_bounds__(256) fz_project_kernel(const __grid_constant__
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
   const int n0 = f.n0, nc1 = f.nc1, np1 = f.np1, n2 = f.n2;
+  grid_dep_launch();
+  grid_dep_wait();
   if (i >= n0 || j >= np1 || k >= n2) return;
   const int nl = n0 * n2, L = i + n0 * k;
   auto phi = [&](int ii, int jj, int kk) { return ld(f.phi, n0, nc1, ii, jj, kk); };
@@ -760,11 +762,10 @@ void launch_fz_update_div(const FzUpdateDiv<T>& f, cudaStream_t st) {
 }
 
 template <typename T>
-void launch_fz_project(const FzProject<T>& f, cudaStream_t st) {
+void launch_fz_project(const FzProject<T>& f, cudaStream_t st, bool chained) {
   const dim3 bs(32, 4, 2);
   const dim3 grid((f.n0 + bs.x - 1) / bs.x, (f.np1 + bs.y - 1) / bs.y, (f.n2 + bs.z - 1) / bs.z);
-  if (f.thermo) fz_project_kernel<T, true><<<grid, bs, 0, st>>>(f);
-  else fz_project_kernel<T, false><<<grid, bs, 0, st>>>(f);
+  launch_chained(f.thermo ? fz_project_kernel<T, true> : fz_project_kernel<T, false>, grid, bs, 0, st, chained, f);
 }
 
 template void launch_fz_momentum<double>(const FzMomentum<double>&, int, cudaStream_t);
@@ -783,7 +784,7 @@ template void launch_fz_energy_walls<double>(const FzEnergy<double>&, int, doubl
 template void launch_fz_energy_walls<float>(const FzEnergy<float>&, int, float*, cudaStream_t);
 template void launch_fz_update_div<double>(const FzUpdateDiv<double>&, cudaStream_t);
 template void launch_fz_update_div<float>(const FzUpdateDiv<float>&, cudaStream_t);
-template void launch_fz_project<double>(const FzProject<double>&, cudaStream_t);
-template void launch_fz_project<float>(const FzProject<float>&, cudaStream_t);
+template void launch_fz_project<double>(const FzProject<double>&, cudaStream_t, bool);
+template void launch_fz_project<float>(const FzProject<float>&, cudaStream_t, bool);
 
 }  // namespace chs

@@ -193,7 +193,7 @@ struct FzProject {
   const double* bulk;
 };
 template <typename T>
-void launch_fz_project(const FzProject<T>& f, cudaStream_t st);
+void launch_fz_project(const FzProject<T>& f, cudaStream_t st, bool chained);
 
 // Poisson right-hand side coeff * (d/dx ux' + d/dy uy' + d/dz uz') of the advanced fields of the momentum
 // step, u' = u with the mass-flux mean subtracted in x and the y wall rows of uy set to v0 / v1: the
@@ -214,5 +214,4 @@ struct FzUpdateDiv {
 };
 template <typename T>
 void launch_fz_update_div(const FzUpdateDiv<T>& f, cudaStream_t st);
-
 }  // namespace chs

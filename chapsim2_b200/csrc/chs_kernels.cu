@@ -1051,6 +1051,7 @@ __global__ void cfft_axis_kernel(const __grid_constant__ FftPlan fp, C* __restri
 
 template <typename R, typename C>
 void launch_rfft_x(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream_t st) {
+  if (fp.rst) return launch_rfft_rows<R, C>(fp, in, out, nrows, st);
   const int lpc = fft_lines_per_cta(fp.n);
   const int npairs = (nrows + 1) / 2;
   const size_t shm = 2 * (size_t)lpc * fp.n * sizeof(C);
@@ -1059,7 +1060,8 @@ void launch_rfft_x(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream
 }
 
 template <typename R, typename C>
-void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st) {
+void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st, bool chained) {
+  if (fp.rst) return launch_irfft_rows<R, C>(fp, in, out, nrows, scale, st, chained);
   const int lpc = fft_lines_per_cta(fp.n);
   const int npairs = (nrows + 1) / 2;
   const size_t shm = 2 * (size_t)lpc * fp.n * sizeof(C);
@@ -1069,13 +1071,14 @@ void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double sc
 template void launch_rfft_x<double, double2>(const FftPlan&, const double*, double2*, int, cudaStream_t);
 template void launch_rfft_x<float, double2>(const FftPlan&, const float*, double2*, int, cudaStream_t);
 template void launch_rfft_x<float, float2>(const FftPlan&, const float*, float2*, int, cudaStream_t);
-template void launch_irfft_x<double, double2>(const FftPlan&, const double2*, double*, int, double, cudaStream_t);
-template void launch_irfft_x<float, double2>(const FftPlan&, const double2*, float*, int, double, cudaStream_t);
-template void launch_irfft_x<float, float2>(const FftPlan&, const float2*, float*, int, double, cudaStream_t);
+template void launch_irfft_x<double, double2>(const FftPlan&, const double2*, double*, int, double, cudaStream_t, bool);
+template void launch_irfft_x<float, double2>(const FftPlan&, const double2*, float*, int, double, cudaStream_t, bool);
+template void launch_irfft_x<float, float2>(const FftPlan&, const float2*, float*, int, double, cudaStream_t, bool);
 
 template <typename C>
 void launch_cfft_axis(const FftPlan& fp, C* data, int na, int nb, int64_t bstride, int64_t stride, int sign,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool chained) {
+  if (fp.rst) return launch_cfft_lines<C>(fp, data, na, nb, bstride, stride, sign, st, chained);
   const int lpc = fft_lines_per_cta(fp.n);
   const int64_t nlines = (int64_t)na * nb;
   const size_t shm = 2 * (size_t)lpc * (fp.n + 1) * sizeof(C);
@@ -1083,8 +1086,8 @@ void launch_cfft_axis(const FftPlan& fp, C* data, int na, int nb, int64_t bstrid
   cfft_axis_kernel<C><<<(unsigned)((nlines + lpc - 1) / lpc), 256, shm, st>>>(fp, data, na, nb, bstride, stride,
                                                                                sign, lpc);
 }
-template void launch_cfft_axis<double2>(const FftPlan&, double2*, int, int, int64_t, int64_t, int, cudaStream_t);
-template void launch_cfft_axis<float2>(const FftPlan&, float2*, int, int, int64_t, int64_t, int, cudaStream_t);
+template void launch_cfft_axis<double2>(const FftPlan&, double2*, int, int, int64_t, int64_t, int, cudaStream_t, bool);
+template void launch_cfft_axis<float2>(const FftPlan&, float2*, int, int, int64_t, int64_t, int, cudaStream_t, bool);
 
 // ===========================================================================
 // FISHPACK y solve: TRID0 (src/poisson_fishpack.f90:20-57) per (kx, kz) on complex data
@@ -1128,9 +1131,6 @@ void launch_ysolve_factor(double* Zr, double* D, int nxh, int ny, int nz, const 
   ysolve_factor_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(Zr, D, nxh, ny, nz, pa, pb, pc, lamx, lamz);
 }
 
-// One CTA per `lt` consecutive (kx, kz) columns: the columns and their precomputed factors are
-// staged in shared memory with coalesced row loads by all threads (eight loads in flight per
-// thread), swept by `lt` threads (one column each), and written back.
 // The spectrum is double2 (FP64 path) or float2 (the FP32 spectrum of the mixed-precision path); the
 // solve itself always runs in FP64.
 __device__ __forceinline__ double2 to_d2(double2 v) { return v; }
@@ -1142,84 +1142,95 @@ __device__ __forceinline__ double2 from_d2<double2>(double2 v) { return v; }
 template <>
 __device__ __forceinline__ float2 from_d2<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
 
+// Columns of up to 160 rows: a CTA owns 16 consecutive columns, lane 2 l + part the real or imaginary part
+// of column l (the system is real), warp w rows w R .. w R + R - 1, all in registers.  A piece is swept twice in
+// each direction: from zero, for its end value and the product of its multipliers, then, once the value
+// entering it is known from the pieces before it, with TRID0's recurrences from that value.  One
+// thread per column swept the tile it replaces from shared memory (16 of 128 threads busy); the whole
+// solve in flight instead takes FP64 128x96x128 from 16.5 to 12.4 us, with an FP32 spectrum to 10.4.
 template <typename C>
-__global__ void __launch_bounds__(128) ysolve_kernel(C* __restrict__ data, int nxh, int ny, int nz,
-                                                     const double* __restrict__ Zr, const double* __restrict__ D,
-                                                     const double* __restrict__ pa, int lt) {
-  extern __shared__ __align__(16) double2 sT[];  // [ny][lt] right-hand sides / solution
-  double2* sF = sT + (size_t)ny * lt;            // [ny][lt] (Zr, D) pairs
-  const int tid = threadIdx.x;
-  const int l = tid % lt;
-  const int64_t nl = (int64_t)nxh * nz;
-  const int64_t g = (int64_t)blockIdx.x * lt + l;
+struct RealOf;
+template <>
+struct RealOf<double2> { using S = double; };
+template <>
+struct RealOf<float2> { using S = float; };
+constexpr int kYsWarps = 16;
+
+template <typename C, int R>
+__global__ void __launch_bounds__(kYsWarps * 32, R == 8 ? 2 : 1)
+    ysolve_kernel(C* __restrict__ data, int nxh, int ny, int nz, const double* __restrict__ Zr,
+                  const double* __restrict__ D, const double* __restrict__ pa) {
+  using S = typename RealOf<C>::S;
+  __shared__ double sE[kYsWarps][32], sM[kYsWarps][32];  // ends of the pieces, products of their multipliers
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5, j0 = w * R;
+  const int64_t nl = (int64_t)nxh * nz, g = (int64_t)blockIdx.x * 16 + (lane >> 1);
   const bool ok = g < nl;
-  const int kz = ok ? (int)(g / nxh) : 0;
-  const int kx = ok ? (int)(g - (int64_t)kz * nxh) : 0;
+  const int64_t gg = ok ? g : nl - 1;
+  const int kz = (int)(gg / nxh), kx = (int)(gg - (int64_t)kz * nxh);
   const int64_t base = (int64_t)kz * ny * nxh + kx;
-  C* col = data + base;
-  const int jstep = blockDim.x / lt;
-  if (ok) {
-    for (int j0 = tid / lt; j0 < ny; j0 += 4 * jstep) {
-      double2 v[4];
-      double z[4], d[4];
+  S* col = reinterpret_cast<S*>(data + base) + (lane & 1);
+  double r[R], A[R], d[R];
+  grid_dep_launch();
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = j0 + u * jstep;
-        if (j < ny) {
-          v[u] = to_d2(col[(int64_t)j * nxh]);
-          z[u] = Zr[base + (int64_t)j * nxh];
-          d[u] = D[base + (int64_t)j * nxh];
-        }
-      }
+  for (int u = 0; u < R; ++u) {
+    const int64_t o = (int64_t)min(j0 + u, ny - 1) * nxh;
+    A[u] = Zr[base + o];
+    d[u] = D[base + o];
+  }
+  grid_dep_wait();  // the factors do not change; the columns are the predecessor's
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = j0 + u * jstep;
-        if (j < ny) {
-          sT[j * lt + l] = v[u];
-          sF[j * lt + l] = make_double2(z[u], d[u]);
-        }
-      }
-    }
+  for (int u = 0; u < R; ++u) r[u] = (double)col[2 * (int64_t)min(j0 + u, ny - 1) * nxh];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const int j = j0 + u;
+    double z = A[u];
+    // the last row's entry is its pivot, zero for the singular system, whose last unknown is pinned to zero
+    if (j == ny - 1) z = z != 0.0 ? 1.0 / z : 0.0;
+    if (j >= ny) { z = 0.0; d[u] = 0.0; }
+    A[u] = __ldg(pa + min(j, ny - 1)) * z;  // pa[0] = 0
+    r[u] *= z;
+  }
+  // forward: T_j = r_j - A_j T_{j-1}
+  double e = 0.0, m = 1.0;
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    e = r[u] - A[u] * e;
+    m *= -A[u];
+  }
+  sE[w][lane] = e;
+  sM[w][lane] = m;
+  __syncthreads();
+  double t = 0.0;
+#pragma unroll 4
+  for (int q = 0; q < w; ++q) t = sE[q][lane] + sM[q][lane] * t;
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    t = r[u] - A[u] * t;
+    r[u] = t;
+  }
+  // backward: x_j = T_j - D_j x_{j+1}
+  e = 0.0;
+  m = 1.0;
+#pragma unroll
+  for (int u = R - 1; u >= 0; --u) {
+    e = r[u] - d[u] * e;
+    m *= -d[u];
   }
   __syncthreads();
-  if (tid < lt && ok) {
-    double2* T = sT + l;
-    const double2* F = sF + l;
-    double2 tp = T[0];
-    const double Z0 = F[0].x;
-    tp.x *= Z0; tp.y *= Z0;
-    T[0] = tp;
-    for (int j = 1; j < ny - 1; ++j) {
-      const double z = F[j * lt].x, a = pa[j];
-      double2 v = T[j * lt];
-      v.x = (v.x - a * tp.x) * z;
-      v.y = (v.y - a * tp.y) * z;
-      T[j * lt] = v;
-      tp = v;
-    }
-    const double zl = F[(ny - 1) * lt].x;
-    double2 v = T[(ny - 1) * lt];
-    // TRID0's singular-pivot pin: the last unknown is zero when the pivot vanishes
-    if (zl != 0.0) {
-      v.x = (v.x - pa[ny - 1] * tp.x) / zl;
-      v.y = (v.y - pa[ny - 1] * tp.y) / zl;
-    } else {
-      v.x = 0.0;
-      v.y = 0.0;
-    }
-    T[(ny - 1) * lt] = v;
-    for (int j = ny - 2; j >= 0; --j) {
-      const double d = F[j * lt].y;
-      double2 u = T[j * lt];
-      u.x = u.x - d * v.x;
-      u.y = u.y - d * v.y;
-      T[j * lt] = u;
-      v = u;
-    }
-  }
+  sE[w][lane] = e;
+  sM[w][lane] = m;
   __syncthreads();
-  if (ok)
-    for (int j = tid / lt; j < ny; j += jstep) col[(int64_t)j * nxh] = from_d2<C>(sT[j * lt + l]);
+  t = 0.0;
+#pragma unroll 4
+  for (int q = W - 1; q > w; --q) t = sE[q][lane] + sM[q][lane] * t;
+#pragma unroll
+  for (int u = R - 1; u >= 0; --u) {
+    t = r[u] - d[u] * t;
+    r[u] = t;
+  }
+#pragma unroll
+  for (int u = 0; u < R; ++u)
+    if (ok && j0 + u < ny) col[2 * (int64_t)(j0 + u) * nxh] = (S)r[u];
 }
 
 // The same solve with one thread per (kx, kz) line working in place in global memory: at a fixed
@@ -1232,6 +1243,8 @@ __global__ void __launch_bounds__(128) ysolve_lines_kernel(C* __restrict__ data,
                                                            const double* __restrict__ Zr,
                                                            const double* __restrict__ D,
                                                            const double* __restrict__ pa) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (int64_t)nxh * nz) return;
   const int kz = (int)(g / nxh), kx = (int)(g - (int64_t)kz * nxh);
@@ -1301,36 +1314,30 @@ __global__ void __launch_bounds__(128) ysolve_lines_kernel(C* __restrict__ data,
 
 template <typename C>
 void launch_ysolve(C* data, int nxh, int ny, int nz, const double* Zr, const double* D, const double* pa,
-                   cudaStream_t st) {
+                   cudaStream_t st, bool chained) {
   if (ny < 2) throw std::runtime_error("ysolve: ny must be at least 2");
+  const int64_t n = (int64_t)nxh * nz;
+  // 16 rows a thread at 256 rows: 191 us at 384x256x384 in FP32 against 176 by the lines kernel
+  const int R = ny <= 8 * kYsWarps ? 8 : 16;
   if (ny > 160) {
-    // tall columns: the shared-memory tile leaves too few solving threads per SM
-    const int64_t n = (int64_t)nxh * nz;
-    ysolve_lines_kernel<C><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(data, nxh, ny, nz, Zr, D, pa);
+    launch_chained(ysolve_lines_kernel<C>, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, st, chained, data, nxh, ny, nz,
+                   Zr, D, pa);
     return;
   }
-  // 16 columns per CTA: a CTA's load, sweep and store phases run one after another, so several
-  // CTAs per SM are needed to keep loads in flight while others sweep
-  int lt = 16;
-  while (lt > 4 && (size_t)ny * lt * 32 > 110 * 1024) lt /= 2;
-  const size_t shm = (size_t)ny * lt * 32;
-  if (shm > 200 * 1024) throw std::runtime_error("ysolve: ny too large for the shared-memory tile");
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(ysolve_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
-  }
-  const int64_t n = (int64_t)nxh * nz;
-  ysolve_kernel<C><<<(unsigned)((n + lt - 1) / lt), 128, shm, st>>>(data, nxh, ny, nz, Zr, D, pa, lt);
+  const unsigned blocks = (unsigned)((n + 15) / 16), threads = (unsigned)((ny + R - 1) / R * 32);
+  launch_chained(R == 8 ? ysolve_kernel<C, 8> : ysolve_kernel<C, 16>, dim3(blocks), dim3(threads), 0, st, chained, data,
+                 nxh, ny, nz, Zr, D, pa);
 }
 template void launch_ysolve<double2>(double2*, int, int, int, const double*, const double*, const double*,
-                                     cudaStream_t);
+                                     cudaStream_t, bool);
 template void launch_ysolve<float2>(float2*, int, int, int, const double*, const double*, const double*,
-                                    cudaStream_t);
+                                    cudaStream_t, bool);
 
 __global__ void spectral_divide_kernel(double2* __restrict__ data, int nxh, int ny, int nz,
                                        const double* __restrict__ k2x, const double* __restrict__ k2y,
                                        const double* __restrict__ k2z, double norm) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int64_t n = (int64_t)nxh * ny * nz;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (int64_t)gridDim.x * blockDim.x) {
     const int kx = (int)(g % nxh);
@@ -1348,8 +1355,8 @@ __global__ void spectral_divide_kernel(double2* __restrict__ data, int nxh, int 
 }
 
 void launch_spectral_divide(double2* data, int nxh, int ny, int nz, const double* k2x, const double* k2y,
-                            const double* k2z, double norm, cudaStream_t st) {
-  spectral_divide_kernel<<<148 * 8, 256, 0, st>>>(data, nxh, ny, nz, k2x, k2y, k2z, norm);
+                            const double* k2z, double norm, cudaStream_t st, bool chained) {
+  launch_chained(spectral_divide_kernel, dim3(148 * 8), dim3(256), 0, st, chained, data, nxh, ny, nz, k2x, k2y, k2z, norm);
 }
 
 // ===========================================================================

@@ -124,7 +124,39 @@ struct FftPlan {
   int radix[16];
   const double2* tw;  // exp(-2 pi i m / n), m = 0..n-1 (device)
   const float2* twf;  // the same rounded to FP32 (device; the FP32 spectrum of the mixed form), or null
+  int rst, rrad[3];   // the register stages of chs_fft.cu (fft_stages), 0: none
 };
+// the register stages of fp.n, if at most three radices make it up
+void fft_stages(FftPlan& fp);
+// the transforms below for plans with register stages (chs_fft.cu)
+template <typename R, typename C>
+void launch_rfft_rows(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream_t st);
+template <typename R, typename C>
+void launch_irfft_rows(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st, bool chained);
+template <typename C>
+void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstride, int64_t stride, int sign,
+                       cudaStream_t st, bool chained);
+
+// Chained launches: a kernel that calls grid_dep_wait() before it touches what its predecessor in the stream wrote, and
+// whose predecessor calls grid_dep_launch() early, may be launched with `chained`, so that its CTAs are set up
+// while the predecessor drains (programmatic dependent launch).  Not behind an event or as a graph's first node.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, bool chained,
+                           const A&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = shm;
+  c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
 
 // real x-lines (rows of length nx, R = double or float) -> half spectra (rows of nx/2+1) of
 // complex type C (double2: FP64 transforms; float2: FP32 transforms of float rows)
@@ -132,12 +164,13 @@ template <typename R, typename C>
 void launch_rfft_x(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream_t st);
 // half spectra -> real x-lines, scaled by `scale`
 template <typename R, typename C>
-void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st);
+void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st,
+                    bool chained = false);
 // complex FFT along a strided axis: element (line, p) at base(line) + p*stride,
 // line = a + na*b with base = a + b*bstride (a fastest); sign -1 forward, +1 backward
 template <typename C>
 void launch_cfft_axis(const FftPlan& fp, C* data, int na, int nb, int64_t bstride, int64_t stride, int sign,
-                      cudaStream_t st);
+                      cudaStream_t st, bool chained = false);
 // forward-sweep factors of the FISHPACK y solve per (kx, kz), computed once (layout (kz, j, kx))
 void launch_ysolve_factor(double* Zr, double* D, int nxh, int ny, int nz, const double* pa, const double* pb,
                           const double* pc, const double* lamx, const double* lamz, cudaStream_t st);
@@ -145,7 +178,7 @@ void launch_ysolve_factor(double* Zr, double* D, int nxh, int ny, int nz, const 
 // FP64 on a double2 or float2 spectrum
 template <typename C>
 void launch_ysolve(C* data, int nxh, int ny, int nz, const double* Zr, const double* D, const double* pa,
-                   cudaStream_t st);
+                   cudaStream_t st, bool chained = false);
 // poisson_010 y stage per (kx, kz) column: reordering, y FFT, cosine post-processing, the
 // pentadiagonal solves (ptab: per system s = 0 odd / 1 even cosine modes and row r < ny/2 the
 // rows [6][ny/2] sub-2, sub-1, t1, t2, super-1, super-2 with main diagonal
@@ -161,7 +194,7 @@ void launch_dct_y_factor(double* pfac, int nxh, int nz, int ny, const double* k2
                          const double* ptab, cudaStream_t st);
 // 3D spectral division by -(kx'^2 + ky'^2 + kz'^2) (zero mode -> 0), with normalisation
 void launch_spectral_divide(double2* data, int nxh, int ny, int nz, const double* k2x, const double* k2y,
-                            const double* k2z, double norm, cudaStream_t st);
+                            const double* k2z, double norm, cudaStream_t st, bool chained = false);
 
 // ---- elementwise and reductions (T = double, or float in the mixed-precision form) ----
 // rhs1 <- dt*(gamma*rhs1 + zeta*rhs0 + alpha*pfc); rhs0 <- old rhs1

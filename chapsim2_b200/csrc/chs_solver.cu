@@ -89,6 +89,7 @@ FftPlan make_fft(int n, std::vector<double2>& tw_host) {
   while (m % 2 == 0) { fp.radix[fp.nst++] = 2; m /= 2; }
   while (m % 3 == 0) { fp.radix[fp.nst++] = 3; m /= 3; }
   if (m != 1) throw std::runtime_error("FFT length must be of the form 2^a 3^b");
+  fft_stages(fp);
   tw_host.resize(n);
   const double pi = 3.141592653589793238462643383279502884;
   for (int k = 0; k < n; ++k) tw_host[k] = make_double2(std::cos(2.0 * pi * k / n), -std::sin(2.0 * pi * k / n));
@@ -1195,11 +1196,17 @@ void upload_fz_rows(chs_handle* H) {
   CK(cudaStreamSynchronize(H->st));
 }
 
+// whether launches may be chained: no events between them (profiling) and none left out (class profile)
+bool chains(const chs_handle* H) { return !H->profiling && H->only_kind < 0; }
+
 template <typename T>
 void poisson_device(chs_handle* H, T* rhs) {
   const int nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2];
   const int nxh = nc0 / 2 + 1;
   cudaStream_t st = H->st;
+  // the launches after the first follow each other directly on the stream, except where a profile puts events
+  // between them or leaves some out
+  const bool ch = chains(H);
   const double nreal = (double)nc0 * nc1 * nc2, nspec = (double)nxh * nc1 * nc2;
   if (H->ifft == 2 && sizeof(T) == sizeof(float) && H->fx.twf && H->fz.twf) {
     // mixed form, FISHPACK: the x and z transforms in FP32 on an FP32 spectrum, the y solve (the
@@ -1207,10 +1214,10 @@ void poisson_device(chs_handle* H, T* rhs) {
     float2* sp = reinterpret_cast<float2*>(H->spec);
     const double b_r2c = 4.0 * nreal + 8.0 * nspec, b_c2c = 16.0 * nspec;
     PROF(H, 1, b_r2c, launch_rfft_x(H->fx, rhs, sp, nc1 * nc2, st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, sp, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st));
-    PROF(H, 2, 32.0 * nspec, launch_ysolve(sp, nxh, nc1, nc2, H->yzr, H->yd, H->pa, st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, sp, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st));
-    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, sp, rhs, nc1 * nc2, 1.0 / ((double)nc0 * (double)nc2), st));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, sp, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st, ch));
+    PROF(H, 2, 32.0 * nspec, launch_ysolve(sp, nxh, nc1, nc2, H->yzr, H->yd, H->pa, st, ch));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, sp, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st, ch));
+    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, sp, rhs, nc1 * nc2, 1.0 / ((double)nc0 * (double)nc2), st, ch));
     H->launches += 5;
     return;
   }
@@ -1218,29 +1225,29 @@ void poisson_device(chs_handle* H, T* rhs) {
   PROF(H, 1, b_r2c, launch_rfft_x(H->fx, rhs, H->spec, nc1 * nc2, st));
   if (H->ifft == 2) {
     // fishpack_fft_simple (src/poisson_fishpack.f90:354-490)
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st));
-    PROF(H, 2, 48.0 * nspec, launch_ysolve(H->spec, nxh, nc1, nc2, H->yzr, H->yd, H->pa, st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st));
-    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0 / ((double)nc0 * (double)nc2), st));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st, ch));
+    PROF(H, 2, 48.0 * nspec, launch_ysolve(H->spec, nxh, nc1, nc2, H->yzr, H->yd, H->pa, st, ch));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st, ch));
+    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0 / ((double)nc0 * (double)nc2), st, ch));
     H->launches += 5;
   } else if (!H->periodic_y) {
     // poisson_010 (src/poisson_1stderivcomp.f90:1457-1816): x and z transforms around the y
     // stage (the FFT normalisation 1/(nx ny nz) is applied there, after the forward transforms)
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st, ch));
     PROF(H, 2, b_c2c, launch_dct_y(H->fy, H->spec, nxh, nc2, H->ayby, H->k2x, H->k2z, H->k2y, H->ptab, H->pfac,
                                    1.0 / ((double)nc0 * (double)nc1 * (double)nc2), st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st));
-    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0, st));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st, ch));
+    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0, st, ch));
     H->launches += 5;
   } else {
     // poisson_000 (src/poisson_1stderivcomp.f90:1016-1195)
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fy, H->spec, nxh, nc2, (int64_t)nxh * nc1, nxh, -1, st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fy, H->spec, nxh, nc2, (int64_t)nxh * nc1, nxh, -1, st, ch));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, -1, st, ch));
     PROF(H, 3, b_c2c, launch_spectral_divide(H->spec, nxh, nc1, nc2, H->k2x, H->k2y, H->k2z,
-                                             1.0 / ((double)nc0 * (double)nc1 * (double)nc2), st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st));
-    PROF(H, 1, b_c2c, launch_cfft_axis(H->fy, H->spec, nxh, nc2, (int64_t)nxh * nc1, nxh, +1, st));
-    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0, st));
+                                             1.0 / ((double)nc0 * (double)nc1 * (double)nc2), st, ch));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fz, H->spec, nxh, nc1, nxh, (int64_t)nxh * nc1, +1, st, ch));
+    PROF(H, 1, b_c2c, launch_cfft_axis(H->fy, H->spec, nxh, nc2, (int64_t)nxh * nc1, nxh, +1, st, ch));
+    PROF(H, 1, b_r2c, launch_irfft_x(H->fx, H->spec, rhs, nc1 * nc2, 1.0, st, ch));
     H->launches += 7;
   }
 }
@@ -1549,15 +1556,13 @@ bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz,
   return true;
 }
 
-// The Poisson right-hand side with the momentum advance folded in (FzUpdateDiv); launch false:
-// only whether it can run.
+// The Poisson right-hand side of the momentum pass's advanced fields; false: no fused form.
 template <typename T>
-bool fused_update_div(chs_handle* H, int isub, double* ux, int w0, int w1, bool launch) {
-  if (!H->kfuse || H->iacc != ACC_CD2 || !H->fz_rows) return false;
+bool fused_div_form(chs_handle* H, int isub, double* ux, int w0, int w1, FzUpdateDiv<T>& F) {
+  if (!H->kfuse || H->iacc != ACC_CD2 || !H->fz_rows || H->periodic_y) return false;
   auto A = [](double* p) { return reinterpret_cast<T*>(p); };
   const auto& B = H->ibc;
   FzBuild b{H};
-  FzUpdateDiv<T> F{};
   F.n0 = H->nc[0]; F.nc1 = H->nc[1]; F.np1 = H->np[1]; F.n2 = H->nc[2];
   F.ux = A(H->mx); F.uy = A(H->my); F.uz = A(H->mz);
   if (!advances_x<T>(H)) { F.ux = A(ux); F.mx = A(H->mx); }
@@ -1572,13 +1577,7 @@ bool fused_update_div(chs_handle* H, int isub, double* ux, int w0, int w1, bool 
   F.rows = H->fz_rows;
   F.out = A(H->pcor);
   F.coeff = 1.0 / (H->tAlpha[isub] * H->sigma2p * H->dt);
-  if (!b.ok || H->periodic_y) return false;
-  if (!launch) return true;
-  const double nf = (double)sizeof(T) * H->n_ccc;
-  PROFD(H, 4, nf * (F.mx ? 5.0 : 4.0), bufs(F.mx ? ux : nullptr, H->mx, H->my, H->mz, H->fb_visc2, F.bulk), bufs(H->pcor),
-        launch_fz_update_div<T>(F, st));
-  H->launches++;
-  return true;
+  return b.ok;
 }
 
 // Energy equation in four launches (wall gradients, fused energy pass, property update, wall
@@ -1696,12 +1695,14 @@ bool fused_project(chs_handle* H, int isub, double* ux, double* uy, double* uz, 
   F.mx = A(H->mx); F.my = A(H->my); F.mz = A(H->mz);
   F.bulk = H->idriven == 1 ? H->scal + 0 : nullptr;
   if (!launch) return true;
+  // it follows the Poisson solve, whose last launch is a barrier of the schedule, directly on the same stream
+  const bool chained = chains(H);
   const double nf = (double)sizeof(T) * H->n_ccc;
   PROFD(H, 3, nf * (TH ? 13.0 : 9.0),
         bufs(H->pcor, H->fb_pr, TH ? H->dDens : nullptr, TH ? H->fb_d : nullptr, upd ? H->mx : nullptr,
              upd ? H->my : nullptr, upd ? H->mz : nullptr, upd ? F.bulk : nullptr, upd ? H->fb_visc2 : nullptr),
         bufs(H->pres, ux, uy, uz, TH ? H->qx : nullptr, TH ? H->qy : nullptr, TH ? H->qz : nullptr),
-        launch_fz_project<T>(F, st));
+        launch_fz_project<T>(F, st, chained));
   H->launches++;
   return true;
 }
@@ -1739,7 +1740,8 @@ void substep_body_t(chs_handle* H, int isub, int parts) {
   const int w0 = B[1][V_QY][0] == BC_DIRICHLET, w1 = B[1][V_QY][1] == BC_DIRICHLET;
   // fused path: the momentum advance u += m - bulk is not stored by itself but formed where the
   // Poisson right-hand side and the projection read u (both fused kernels must be available)
-  const bool defer = fused_update_div<T>(H, isub, ux, w0, w1, false) &&
+  FzUpdateDiv<T> F{};
+  const bool defer = fused_div_form<T>(H, isub, ux, w0, w1, F) &&
                      fused_project<T>(H, isub, ux, uy, uz, w0, w1, true, false);
   const bool mom_fused = fused_momentum<T>(H, isub, ux, uy, uz, defer);
   const bool upd = defer && mom_fused;
@@ -1904,7 +1906,10 @@ void substep_body_t(chs_handle* H, int isub, int parts) {
   // Update_thermal_properties has already set rho_m1 = rho, so the term is zero and left out.
   const double coeff = 1.0 / (H->tAlpha[isub] * H->sigma2p * H->dt);
   if (upd) {
-    fused_update_div<T>(H, isub, ux, w0, w1, true);
+    PROFD(H, 4, (double)sizeof(T) * H->n_ccc * (F.mx ? 5.0 : 4.0),
+          bufs(F.mx ? ux : nullptr, H->mx, H->my, H->mz, H->fb_visc2, F.bulk), bufs(H->pcor),
+          launch_fz_update_div<T>(F, st));
+    H->launches++;
   } else {
     std::vector<OpTerm<T>> t = {term<T>(0, D1P2C, bx_qx, any, src(A(ux)), s_pcc, coeff, 0),
                                 term<T>(1, D1P2C, by_qy, nullptr, src(A(uy)), s_cpc, coeff, 0),

@@ -101,6 +101,7 @@ bool radix_plan(int n, FftPlan& fp) {
   while (m % 4 == 0) { fp.radix[fp.nst++] = 4; m /= 4; }
   while (m % 2 == 0) { fp.radix[fp.nst++] = 2; m /= 2; }
   while (m % 3 == 0) { fp.radix[fp.nst++] = 3; m /= 3; }
+  fft_stages(fp);
   return m == 1;
 }
 

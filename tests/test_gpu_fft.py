@@ -1,0 +1,72 @@
+"""Transforms of the Poisson solvers at every shape of their stage plan (one to three register stages with each
+radix, lengths beyond them, odd lengths, ragged line counts) through the periodic solver against
+numpy's FFT, the y solve at the ends of its piece sizes, and the FP32 spectrum of the mixed form against the
+FP64 path."""
+import numpy as np
+import pytest
+
+from chapsim2_b200 import config as C
+from chapsim2_b200 import initial as I
+from chapsim2_b200 import solver as S
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [8, 9, 12, 16, 18, 24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128, 144, 162, 192, 216, 243, 256, 288, 324,
+           384, 432, 486, 512, 576, 648, 729, 768, 1024]
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_lengths(n):
+    for axis in range(3):
+        nc = [18, 9, 12]
+        nc[axis] = n
+        cfg = C.taylor_green(16, iacc=C.IACCU_CD2)
+        cfg.nc = tuple(nc)
+        g = S.Solver(cfg)
+        rhs = np.random.default_rng(n).standard_normal((nc[2], nc[1], nc[0]))
+        got = g.solve_fft_poisson(rhs)
+        g.close()
+        h = (cfg.lxx / nc[0], (cfg.lyt - cfg.lyb) / nc[1], cfg.lzz / nc[2])
+        k2 = [(2.0 / h[d] * np.sin(np.pi * np.arange(nc[d]) / nc[d])) ** 2 for d in range(3)]
+        k2 = k2[2][:, None, None] + k2[1][None, :, None] + k2[0][None, None, :]
+        f = np.fft.fftn(rhs)
+        k2[0, 0, 0] = 1.0
+        f /= -k2
+        f[0, 0, 0] = 0.0
+        ref = np.fft.ifftn(f).real
+        # error growth of an FFT is O(eps log n); five passes over values of the result's size
+        assert np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max(), axis
+
+
+@pytest.mark.parametrize("ny", [8, 9, 15, 16, 17, 127, 128, 129, 160, 255, 256, 257])
+def test_y_solve(ny):
+    cfg = C.channel(nc=(18, ny, 12), iacc=1)
+    o, g = po.Oracle(cfg), S.Solver(cfg)
+    rhs = np.random.default_rng(ny).standard_normal(o.shape_ccc)
+    rhs -= rhs.mean(axis=(0, 2), keepdims=True)
+    # the mean mode's last pivot is zero up to round-off, so its constant is round-off too where it is not pinned
+    ref, got = [a - a.mean() for a in (o.poisson(rhs), g.solve_fft_poisson(rhs))]
+    assert np.abs(ref - got).max() / np.abs(ref).max() < 1e-11
+    g.close()
+
+
+@pytest.mark.parametrize("nc", [(8, 9, 16), (54, 17, 108), (162, 24, 8), (18, 130, 256), (384, 12, 24)])
+def test_fp32_spectrum(nc):
+    cfg = C.channel(nc=nc, iacc=1, dt=1e-3)
+    f = I.channel_fields(cfg)
+    res = []
+    for prec in (S.CHS_FP64, S.CHS_MIXED):
+        g = S.Solver(cfg, precision=prec)
+        g.set_fields(*f)
+        g.Solve_momentum_eq(0)
+        g.step(1)
+        res.append(g.get_fields())
+        g.close()
+    # eps of FP32 times the velocity scale; the pressure's source is a velocity difference over the spacing
+    # and dt, and its inverse Laplacian gains a spacing squared: eps q h / dt for each of four substeps
+    q = max(np.abs(a).max() for a in res[0][:3])
+    for a, b in zip(res[1][:3], res[0][:3]):
+        assert np.abs(a - b).max() <= 1e-5 * q
+    h = max(cfg.lxx / nc[0], cfg.lzz / nc[2])
+    assert np.abs(res[1][3] - res[0][3]).max() <= 4 * 2.0 ** -23 * q * h / cfg.dt
