@@ -188,6 +188,8 @@ struct chs_handle {
   double* pfac = nullptr;                   // and the elimination factors per (kx, |kz|)
   // graphs per substep (1..3) and for a whole step
   cudaGraphExec_t gexec[4] = {nullptr, nullptr, nullptr, nullptr};
+  cudaGraphExec_t gstep = nullptr;
+  long long kernels_per_step = 0;
   // the energy and momentum parts of substeps 1..3 as separate graphs (host-array pipeline)
   cudaGraphExec_t gpart[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
   long long kernels_per_part[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
@@ -1102,6 +1104,7 @@ void setup_device(chs_handle* H, const chs_config* c) {
 }
 
 void drop_graphs(chs_handle* H) {
+  if (H->gstep) { cudaGraphExecDestroy(H->gstep); H->gstep = nullptr; }
   for (auto& g : H->gexec)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   for (auto& row : H->gpart)
@@ -2578,15 +2581,15 @@ void stats_update_t(chs_handle* H, int nstat) {
   H->launches++;
 }
 
-// capture substep isub (parts PART_*) as one graph; returns its kernel count
-long long capture_one(chs_handle* H, int isub, int parts, cudaGraphExec_t* out) {
+// capture the substeps isub0 .. isub1 (parts PART_*) as one graph; returns its kernel count
+long long capture_one(chs_handle* H, int isub0, int isub1, int parts, cudaGraphExec_t* out) {
   cudaGraph_t g;
   const long long before = H->launches;
   CK(cudaStreamBeginCapture(H->st, cudaStreamCaptureModeThreadLocal));
   H->capturing = true;
   try {
     H->dag_start();
-    substep_body(H, isub, parts);
+    for (int isub = isub0; isub <= isub1; ++isub) substep_body(H, isub, parts);
     H->dag_stop();
   } catch (...) {
     H->dag_stop();
@@ -2603,14 +2606,21 @@ long long capture_one(chs_handle* H, int isub, int parts, cudaGraphExec_t* out) 
   return n;
 }
 
+// a whole RK3 step as one graph: no gap between the substeps, whose independent launches overlap
+void run_step(chs_handle* H) {
+  if (!H->gstep) H->kernels_per_step = capture_one(H, 1, 3, PART_ALL, &H->gstep);
+  CK(cudaGraphLaunch(H->gstep, H->st));
+  H->launches += H->kernels_per_step;
+}
+
 void capture_graphs(chs_handle* H) {
-  for (int isub = 1; isub <= 3; ++isub) H->kernels_per_sub[isub] = capture_one(H, isub, PART_ALL, &H->gexec[isub]);
+  for (int isub = 1; isub <= 3; ++isub) H->kernels_per_sub[isub] = capture_one(H, isub, isub, PART_ALL, &H->gexec[isub]);
 }
 
 void capture_part_graphs(chs_handle* H) {
   for (int isub = 1; isub <= 3; ++isub) {
-    H->kernels_per_part[0][isub] = capture_one(H, isub, PART_ENERGY, &H->gpart[0][isub]);
-    H->kernels_per_part[1][isub] = capture_one(H, isub, PART_MOMENTUM, &H->gpart[1][isub]);
+    H->kernels_per_part[0][isub] = capture_one(H, isub, isub, PART_ENERGY, &H->gpart[0][isub]);
+    H->kernels_per_part[1][isub] = capture_one(H, isub, isub, PART_MOMENTUM, &H->gpart[1][isub]);
   }
 }
 
@@ -2703,13 +2713,12 @@ void snapshot(chs_handle* H, char* buf, bool save) {
 }
 
 float time_steps_ms(chs_handle* H, int nsteps) {
-  if (!H->gexec[1]) capture_graphs(H);
+  if (!H->gstep) H->kernels_per_step = capture_one(H, 1, 3, PART_ALL, &H->gstep);
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
   CK(cudaEventRecord(a, H->st));
-  for (int s = 0; s < nsteps; ++s)
-    for (int isub = 1; isub <= 3; ++isub) CK(cudaGraphLaunch(H->gexec[isub], H->st));
+  for (int s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(H->gstep, H->st));
   CK(cudaEventRecord(b, H->st));
   CK(cudaEventSynchronize(b));
   float ms = 0.0f;
@@ -3040,7 +3049,8 @@ int chs_momentum_substep(chs_handle* H, int isub) {
     if (H->thermo) {
       // the captured graphs hold the whole substep (energy + momentum)
       substep_body(H, isub, PART_MOMENTUM);
-    } else if (isub >= 1 && H->gexec[isub]) {
+    } else if (isub >= 1 && (H->gexec[isub] || H->gstep)) {
+      if (!H->gexec[isub]) capture_graphs(H);
       CK(cudaGraphLaunch(H->gexec[isub], H->st));
       H->launches += H->kernels_per_sub[isub];
     } else {
@@ -3053,12 +3063,7 @@ int chs_momentum_substep(chs_handle* H, int isub) {
 int chs_step(chs_handle* H, int nsteps) {
   if (!H) return CHS_ERR_ARG;
   return guard(H, [&] {
-    if (!H->gexec[1]) capture_graphs(H);
-    for (int s = 0; s < nsteps; ++s)
-      for (int isub = 1; isub <= 3; ++isub) {
-        CK(cudaGraphLaunch(H->gexec[isub], H->st));
-        H->launches += H->kernels_per_sub[isub];
-      }
+    for (int s = 0; s < nsteps; ++s) run_step(H);
     CK(cudaGetLastError());
   });
 }
@@ -3094,16 +3099,12 @@ int chs_momentum_substep_host(chs_handle* H, int isub, double* qx, double* qy, d
 int chs_time_steps(chs_handle* H, int nsteps, float* ms) {
   if (!H || !ms || nsteps < 0) return CHS_ERR_ARG;
   return guard(H, [&] {
-    if (!H->gexec[1]) capture_graphs(H);
+    if (!H->gstep) H->kernels_per_step = capture_one(H, 1, 3, PART_ALL, &H->gstep);
     cudaEvent_t a, b;
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     CK(cudaEventRecord(a, H->st));
-    for (int s = 0; s < nsteps; ++s)
-      for (int isub = 1; isub <= 3; ++isub) {
-        CK(cudaGraphLaunch(H->gexec[isub], H->st));
-        H->launches += H->kernels_per_sub[isub];
-      }
+    for (int s = 0; s < nsteps; ++s) run_step(H);
     CK(cudaEventRecord(b, H->st));
     CK(cudaEventSynchronize(b));
     CK(cudaEventElapsedTime(ms, a, b));
@@ -3317,7 +3318,7 @@ int chs_profile_class(chs_handle* H, int isub, int kind, int reps, float* ms) {
     cudaGraphExec_t ge = nullptr;
     H->only_kind = kind;
     try {
-      capture_one(H, isub, PART_ALL, &ge);
+      capture_one(H, isub, isub, PART_ALL, &ge);
     } catch (...) {
       H->only_kind = -1;
       throw;
