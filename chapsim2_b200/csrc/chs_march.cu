@@ -120,33 +120,29 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
     if (wall_from && !z_only) copy_pair(set + kData + 2 * threadIdx.x, wall_from + kw * n0);
   };
 
-  const T half = T(0.5), third = T(1.0 / 3.0), dxi = T(f.dxi), dzi = T(f.dzi), rre = T(f.rre);
+  const T third = T(1.0 / 3.0), dxi = T(f.dxi), dzi = T(f.dzi), rre = T(f.rre), rre2 = T(2.0 * f.rre);
+  const T quarter = T(0.25), rre4 = T(0.25 * f.rre);
   // y weights of row j (cells) and edge j (points)
   auto wcell = [&](int j) { return T(f.wc[PY ? (j + ny) % ny : min(max(j, 0), ny - 1)]); };
   auto wedge = [&](int j) { return T(f.wp[PY ? (j + ny) % ny : min(max(j, 0), np1 - 1)]); };
 #define V(S, F, R, C) (S)[((F) * kRows + (R)) * kXS + (C)]
 
-  // ---- the stresses.  A: the set of plane k (qz, gz: k + 1), B: of k - 1 (qz, gz: k); set row r, column c
+  // ---- the stresses.  A: the set of plane k (qz, gz: k + 1), B: of k - 1 (qz, gz: k); set row r, column c.
+  // Interpolated factors enter as sums of two or four values, their halves in one constant.
   // normal stress a of (xx, yy, zz) at the cell centre
   auto normal = [&](const T* A, const T* B, int r, int c, T wc, int a) -> T {
     const T qx0 = V(A, QX, r, c), qx1 = V(A, QX, r, c + 1), qy0 = V(A, QY, r, c), qy1 = V(A, QY, r + 1, c);
     const T qz0 = V(B, QZ, r, c), qz1 = V(A, QZ, r, c);
     const T dx = dxi * (qx1 - qx0), dy = wc * (qy1 - qy0), dz = dzi * (qz1 - qz0);
     const T d = a == 0 ? dx : (a == 1 ? dy : dz);
-    T v = T(2) * (d - third * (dx + dy + dz));
+    T v = rre2 * (d - third * (dx + dy + dz));
     if (TH) v *= V(A, MU, r, c);
-    T m, q;
-    if (a == 0) {
-      q = half * (qx0 + qx1);
-      m = TH ? half * (V(A, GX, r, c) + V(A, GX, r, c + 1)) : q;
-    } else if (a == 1) {
-      q = half * (qy0 + qy1);
-      m = TH ? half * (V(A, GY, r, c) + V(A, GY, r + 1, c)) : q;
-    } else {
-      q = half * (qz0 + qz1);
-      m = TH ? half * (V(B, GZ, r, c) + V(A, GZ, r, c)) : q;
-    }
-    return rre * v - m * q;
+    const T q = a == 0 ? qx0 + qx1 : (a == 1 ? qy0 + qy1 : qz0 + qz1);
+    T m = q;
+    if (TH)
+      m = a == 0 ? V(A, GX, r, c) + V(A, GX, r, c + 1)
+                 : (a == 1 ? V(A, GY, r, c) + V(A, GY, r + 1, c) : V(B, GZ, r, c) + V(A, GZ, r, c));
+    return v - quarter * m * q;
   };
   // rows r and r - 1 of a y-cell array at edge r; beyond a wall (side 1 below, 2 above) the value that
   // puts the wall's (row q of the wall rows of set Wl) in the middle
@@ -163,58 +159,56 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
   auto edge_xy = [&](const T* A, int r, int c, T wp, int side, T& e0, T& e1) {
     T qh, ql;
     ypair(A, QX, r, c, A, WQX, side, qh, ql);
-    const T qyr = V(A, QY, r, c), qyl = V(A, QY, r, c - 1);
-    const T qxi = half * (qh + ql), qyi = half * (qyr + qyl);
-    T v = wp * (qh - ql) + dxi * (qyr - qyl);
-    T m0 = qyi, m1 = qxi;
+    const T qyr = V(A, QY, r, c), qyl = V(A, QY, r, c - 1), qxs = qh + ql, qys = qyr + qyl;
+    T v = wp * (qh - ql) + dxi * (qyr - qyl), m0 = qys, m1 = qxs;
     if (TH) {
       T mh, ml, nh, nlo, gh, gl;
       ypair(A, MU, r, c, A, WMU, side, mh, ml);
       ypair(A, MU, r, c - 1, A, WMU, side, nh, nlo);
-      v *= half * (half * (mh + ml) + half * (nh + nlo));
+      v *= rre4 * ((mh + ml) + (nh + nlo));
       ypair(A, GX, r, c, A, WG, side, gh, gl);
-      m0 = half * (V(A, GY, r, c) + V(A, GY, r, c - 1));
-      m1 = half * (gh + gl);
+      m0 = V(A, GY, r, c) + V(A, GY, r, c - 1);
+      m1 = gh + gl;
+    } else {
+      v *= rre;
     }
-    v *= rre;
-    e0 = v - m0 * qxi;
-    e1 = v - m1 * qyi;
+    e0 = v - quarter * m0 * qxs;
+    e1 = v - quarter * m1 * qys;
   };
   // xz edge: of the x component (e0) and the z component (e2)
   auto edge_xz = [&](const T* A, const T* B, int r, int c, T& e0, T& e2) {
     const T xa = V(A, QX, r, c), xb = V(B, QX, r, c), zr = V(B, QZ, r, c), zl = V(B, QZ, r, c - 1);
-    const T qxi = half * (xa + xb), qzi = half * (zr + zl);
-    T v = dzi * (xa - xb) + dxi * (zr - zl);
-    T m0 = qzi, m2 = qxi;
+    const T qxs = xa + xb, qzs = zr + zl;
+    T v = dzi * (xa - xb) + dxi * (zr - zl), m0 = qzs, m2 = qxs;
     if (TH) {
-      v *= half * (half * (V(A, MU, r, c) + V(A, MU, r, c - 1)) + half * (V(B, MU, r, c) + V(B, MU, r, c - 1)));
-      m0 = half * (V(B, GZ, r, c) + V(B, GZ, r, c - 1));
-      m2 = half * (V(A, GX, r, c) + V(B, GX, r, c));
+      v *= rre4 * ((V(A, MU, r, c) + V(A, MU, r, c - 1)) + (V(B, MU, r, c) + V(B, MU, r, c - 1)));
+      m0 = V(B, GZ, r, c) + V(B, GZ, r, c - 1);
+      m2 = V(A, GX, r, c) + V(B, GX, r, c);
+    } else {
+      v *= rre;
     }
-    v *= rre;
-    e0 = v - m0 * qxi;
-    e2 = v - m2 * qzi;
+    e0 = v - quarter * m0 * qxs;
+    e2 = v - quarter * m2 * qzs;
   };
   // yz edge: of the y component (e1) and the z component (e2)
   auto edge_yz = [&](const T* A, const T* B, int r, int c, T wp, int side, T& e1, T& e2) {
     T zh, zl;
     ypair(B, QZ, r, c, A, WQZ, side, zh, zl);
-    const T ya = V(A, QY, r, c), yb = V(B, QY, r, c);
-    const T qyi = half * (ya + yb), qzi = half * (zh + zl);
-    T v = wp * (zh - zl) + dzi * (ya - yb);
-    T m1 = qzi, m2 = qyi;
+    const T ya = V(A, QY, r, c), yb = V(B, QY, r, c), qys = ya + yb, qzs = zh + zl;
+    T v = wp * (zh - zl) + dzi * (ya - yb), m1 = qzs, m2 = qys;
     if (TH) {
       T mh, ml, nh, nlo, gh, gl;
       ypair(A, MU, r, c, A, WMU, side, mh, ml);
       ypair(B, MU, r, c, B, WMU, side, nh, nlo);
-      v *= half * (half * (mh + ml) + half * (nh + nlo));
+      v *= rre4 * ((mh + ml) + (nh + nlo));
       ypair(B, GZ, r, c, A, WG, side, gh, gl);
-      m1 = half * (gh + gl);
-      m2 = half * (V(A, GY, r, c) + V(B, GY, r, c));
+      m1 = gh + gl;
+      m2 = V(A, GY, r, c) + V(B, GY, r, c);
+    } else {
+      v *= rre;
     }
-    v *= rre;
-    e1 = v - m1 * qyi;
-    e2 = v - m2 * qzi;
+    e1 = v - quarter * m1 * qys;
+    e2 = v - quarter * m2 * qzs;
   };
   auto side_of = [&](int j) { return PY ? 0 : (j == 0 ? 1 : (j == ny ? 2 : 0)); };
 
