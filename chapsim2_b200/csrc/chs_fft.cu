@@ -8,7 +8,8 @@
 // stage free of bank conflicts; twiddles are read from a copy in shared memory.
 //
 // The kernels of chs_kernels.cu (radix 4, 2, 3 stages through two shared buffers with twiddles from
-// global memory) pass a line through shared memory nst + 1 times; they keep longer lines.
+// global memory) pass a line through shared memory nst + 1 times; they keep longer lines.  The four transforms of a
+// solve, with those and with these: 128x96x128 FP64 54 and 35 us, 384x256x384 FP32 758 and 490, 64^3 (six) 48 and 23.
 #include <cuda_runtime.h>
 
 #include <algorithm>
