@@ -126,6 +126,8 @@ struct FftPlan {
   const float2* twf;  // the same rounded to FP32 (device; the FP32 spectrum of the mixed form), or null
   int rst, rrad[3];   // the register stages of chs_fft.cu (fft_stages), 0: none
 };
+// exp(-2 pi i m / n), m = 0..n-1
+void fft_twiddles(int n, double2* tw);
 // the register stages of fp.n, if at most three radices make it up
 void fft_stages(FftPlan& fp);
 // the transforms below for plans with register stages (chs_fft.cu)

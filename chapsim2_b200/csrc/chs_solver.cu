@@ -91,8 +91,7 @@ FftPlan make_fft(int n, std::vector<double2>& tw_host) {
   if (m != 1) throw std::runtime_error("FFT length must be of the form 2^a 3^b");
   fft_stages(fp);
   tw_host.resize(n);
-  const double pi = 3.141592653589793238462643383279502884;
-  for (int k = 0; k < n; ++k) tw_host[k] = make_double2(std::cos(2.0 * pi * k / n), -std::sin(2.0 * pi * k / n));
+  fft_twiddles(n, tw_host.data());
   return fp;
 }
 

@@ -105,11 +105,6 @@ bool radix_plan(int n, FftPlan& fp) {
   return m == 1;
 }
 
-void twiddles(int n, double2* tw) {
-  const double pi = 3.141592653589793238462643383279502884;
-  for (int k = 0; k < n; ++k) tw[k] = make_double2(std::cos(2.0 * pi * k / n), -std::sin(2.0 * pi * k / n));
-}
-
 // squared modified wavenumbers of the periodic C2P first derivative, as the handle path builds them
 void mod_k2(int n, double len, double dh, int iacc, double* v) {
   const double pi = 2.0 * std::asin(1.0);
@@ -183,7 +178,7 @@ extern "C" int chs_poisson_periodic_static(double* d_rhs, const int nc[3], const
       Staging& sg = *g_stage[dev];
       const FftPlan* fp[3] = {&fx, &fy, &fz};
       for (int d = 0; d < 3; ++d) {
-        twiddles(nc[d], sg.tw[d]);
+        fft_twiddles(nc[d], sg.tw[d]);
         mod_k2(nc[d], len[d], len[d] / nc[d], iacc, sg.k2[d]);
         e = cudaMemcpyAsync(const_cast<double2*>(fp[d]->tw), sg.tw[d], nc[d] * sizeof(double2),
                             cudaMemcpyHostToDevice, st);
