@@ -1,26 +1,29 @@
 // Compact line operators with the line kept in registers (CP4 and CP6).
 //
 // A CTA owns 32 lines.  Warp w holds rows w*R .. w*R + R-1 of every one of them, lane l those of line
-// l, so a thread solves a piece of R rows of one line by itself and the pieces are joined exactly:
+// l, so a thread solves a piece of R rows of one line.  Each direction of the Thomas sweep
 //
-//   forward   y_i = D_i r_i - A_i y_{i-1}   over the piece from y = 0, then y_i += P_i y_in
-//   backward  x_i = y_i - C_i x_{i+1}       over the piece from x = 0, then x_i += Q_i x_out
+//   forward   y_i = (r_i - a_i y_{i-1}) D_i       backward   x_i = y_i - C_i x_{i+1}
 //
-// with D = 1/pivot, A = a/pivot, C = c/pivot the Thomas factors of the line, P_i the product of the
-// -A and Q_i that of the -C between row i and the piece's start or end (line_coefs in chs_plan.cpp).
-// y_in and x_out, the values at the ends of the neighbouring pieces, follow from the pieces' own ends
-// by the same recurrences over at most 16 pieces, which each thread runs for itself from shared
-// memory.  The last row of a periodic line stands outside the Thomas system (its row of factors
-// passes the right-hand side through) and closes it as Solve_TDMA_cyclic does
-// (src/basics_algorithms.f90:60-109).
+// with D = 1/pivot and C = c/pivot (line_coefs in chs_plan.cpp) runs over a piece twice: from zero, for the value at
+// the piece's end, and, once the value entering the piece is known, from that value.  It follows from the ends of the
+// pieces before: end of a piece = its end from zero + (product of its -a D, or -C) times the value entering it, over at
+// most 16 pieces, which each thread runs for itself from shared memory.  The last row of a periodic line stands
+// outside the Thomas system (its row of factors passes the right-hand side through) and closes it as
+// Solve_TDMA_cyclic does (src/basics_algorithms.f90:60-109).
+//
+// The second sweep instead of a correction of every row, y_i += P_i y_in, keeps the rounding of the plain sweep: the
+// corrected rows, with r1 dd and a D as one constant each, erred by up to 1.34 times as much (CP4 differences at 128
+// points, 1.74 and 1.28 units of 2^-53; FP32 velocities of a CP6 channel 4 to 9 % more).
 //
 // What bounds it: with one thread per line (line_op_kernel) a CTA ran two sweeps of n dependent rows
 // in one warp of eight while the others waited, and reached 15 % of the memory rate.  Here every warp
 // sweeps R rows, all R + 3 input values of a thread are in flight at once, and for y and z lines
 // neither input nor output passes through shared memory (32 neighbouring x positions are one 256-byte
 // segment of FP64 at every row); x lines are transposed through a shared tile with an odd stride.
-// Pieces of 8 rows beat 16 (shorter chains, twice the warps): FP64 line solves of a substep, 128x96x128
-// CP6 channel 486 against 593 us (1029 us by line_op_kernel), Taylor-Green 96^3 244 against 322 us.
+// Pieces of 8 rows beat 16 (shorter chains, twice the warps): FP64 line solves of a substep, one sweep and a
+// correction, 128x96x128 CP6 channel 486 against 593 us (1029 us by line_op_kernel), Taylor-Green 96^3 244 against
+// 322 us.  With the second sweep 502 and 248 us.
 #include <cuda_runtime.h>
 
 #include <stdexcept>
@@ -32,7 +35,7 @@ namespace chs {
 
 namespace {
 
-// the factors of one row (line_coefs): d, a | p, c | q, x | m, unused
+// the factors of one row (line_coefs): d, a | c, q | x, m | p, unused
 template <typename T>
 struct Pair2;
 template <>
@@ -43,6 +46,11 @@ struct Pair2<float> { using V = float2; };
 template <typename T>
 __device__ __forceinline__ typename Pair2<T>::V coef2(const T* __restrict__ tab, int row, int k) {
   return __ldg(reinterpret_cast<const typename Pair2<T>::V*>(tab + (size_t)row * kLineCoefs) + k);
+}
+
+template <typename T>
+__device__ __forceinline__ T coef1(const T* __restrict__ tab, int row, int k) {
+  return __ldg(tab + (size_t)row * kLineCoefs + k);
 }
 
 // v[u] = the input expression at the positions at(u), u < N; the modes are switched on once so that the
@@ -134,8 +142,8 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
   // last two rows of a periodic line
   const bool edge = i0 + kLo < 0 || i0 + kLo + N > nin || i0 < P.b_lo || i0 + R - 1 > P.b_hi || i0 + R > nout - 2;
   if (threadIdx.x < W) {
-    sP[threadIdx.x] = coef2(tab, threadIdx.x * R + R - 1, 1).x;
-    sP[W + threadIdx.x] = coef2(tab, threadIdx.x * R, 2).x;
+    sP[threadIdx.x] = coef2(tab, threadIdx.x * R + R - 1, 3).x;
+    sP[W + threadIdx.x] = coef2(tab, threadIdx.x * R, 1).y;
   }
 
   int base = 0, obase = 0, ps = 1;  // first value of the line in the input and output, row stride
@@ -193,11 +201,11 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
   // ---- right-hand side
   T x[R];
   {
-    const T r1 = T(P.r1 * P.dd), r2 = T(P.r2 * P.dd), sg = T(P.sgn);
+    const T r1 = T(P.r1), r2 = T(P.r2), dd = T(P.dd), sg = T(P.sgn);
 #pragma unroll
     for (int u = 0; u < R; ++u)  // row i0 + u; v[u] is row i0 + kLo + u
-      x[u] = CIN ? r1 * (v[u + 2] + sg * v[u + 1]) + r2 * (v[u + 3] + sg * v[u])
-                 : r1 * (sg * v[u + 1] + v[u + 2]) + r2 * (sg * v[u] + v[u + 3]);
+      x[u] = (CIN ? r1 * (v[u + 2] + sg * v[u + 1]) + r2 * (v[u + 3] + sg * v[u])
+                  : r1 * (sg * v[u + 1] + v[u + 2]) + r2 * (sg * v[u] + v[u + 3])) * dd;
   }
   if (edge && !P.lwrap) {
     // boundary rows of a line with ends, at most four
@@ -215,30 +223,27 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
         if (S.row == i0 + u) x[u] = s;
     }
   }
-  // ---- forward piece
+  // ---- end of the forward piece
   {
     T y = T(0);
 #pragma unroll
     for (int u = 0; u < R; ++u) {
-      const auto c = coef2(tab, i0 + u, 0);
-      y = x[u] * c.x - c.y * y;
-      x[u] = y;
+      const auto da = coef2(tab, i0 + u, 0);
+      y = x[u] * da.x - (da.y * da.x) * y;
     }
     sE[w * 32 + lane] = y;
   }
   __syncthreads();
-  // ---- join the forward pieces, backward piece
+  // ---- forward sweep from the joined value, start of the backward piece
   {
     T y = T(0);
 #pragma unroll 4
     for (int m = 0; m < w; ++m) y = sE[m * 32 + lane] + sP[m] * y;
-    T z = T(0);
-    T c[R];
 #pragma unroll
     for (int u = 0; u < R; ++u) {
-      const auto pc = coef2(tab, i0 + u, 1);
-      x[u] += pc.x * y;
-      c[u] = pc.y;
+      const auto da = coef2(tab, i0 + u, 0);
+      y = (x[u] - da.y * y) * da.x;
+      x[u] = y;
     }
     if (edge && P.tdma == 2) {
 #pragma unroll
@@ -247,15 +252,13 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
         if (i0 + u == nout - 1) sN[32 + lane] = x[u];
       }
     }
+    T z = T(0);
 #pragma unroll
-    for (int u = R - 1; u >= 0; --u) {
-      z = x[u] - c[u] * z;
-      x[u] = z;
-    }
+    for (int u = R - 1; u >= 0; --u) z = x[u] - coef1(tab, i0 + u, 2) * z;
     sF[w * 32 + lane] = z;
   }
   __syncthreads();
-  // ---- join the backward pieces, cyclic closure, metric and wall slopes
+  // ---- backward sweep from the joined value, cyclic closure, metric and wall slopes
   {
     const T* sQ = sP + W;
     T z = T(0);
@@ -269,10 +272,13 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
       xn = (sN[32 + lane] - T(P.cn) * x0 - T(P.an) * sN[lane]) * T(P.inv_den);
     }
 #pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const auto c = coef2(tab, i0 + u, 2);
-      x[u] += c.x * z;
-      x[u] += c.y * xn;
+    for (int u = R - 1; u >= 0; --u) {
+      z = x[u] - coef1(tab, i0 + u, 2) * z;
+      x[u] = z;
+    }
+    if (P.tdma == 2) {
+#pragma unroll
+      for (int u = 0; u < R; ++u) x[u] += coef1(tab, i0 + u, 4) * xn;
     }
     if (edge && P.tdma == 2) {
 #pragma unroll
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
     }
     if (P.lmap >= 0) {
 #pragma unroll
-      for (int u = 0; u < R; ++u) x[u] *= coef2(tab, i0 + u, 3).x;
+      for (int u = 0; u < R; ++u) x[u] *= coef1(tab, i0 + u, 5);
     }
     if (edge && (P.neu1 || P.neu2)) {
 #pragma unroll

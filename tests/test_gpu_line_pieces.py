@@ -4,6 +4,7 @@ and one beyond it, which runs the tile kernel) with line counts off the 32 of a 
 which form every input expression and store mode, against the oracle's."""
 import numpy as np
 import pytest
+import scipy.fft as sf
 
 from chapsim2_b200 import config as C
 from chapsim2_b200 import initial as I
@@ -81,4 +82,28 @@ def test_substep(case, nc, precision):
     assert np.abs(got[3] - ref[3]).max() <= 500 * eps * q
     if tc is not None:
         assert np.abs(g.get_thermo()["T"] - o.get_thermo()["T"]).max() <= eps
+    g.close()
+
+
+@pytest.mark.parametrize("acc,bound", [(3, (1.4, 1.4)), (4, (1.8, 1.75))])
+@pytest.mark.parametrize("n", [64, 128, 144, 256, 288, 384])
+def test_error(n, acc, bound):
+    """Error of the x operators against their Fourier symbol in extended precision, rms in units of 2^-53: a right-hand side
+    of four roundings and the sweeps' two, one and one, as one thread sweeping the whole line makes them, come to 1.3 and
+    1.15 (CP4 derivative, interpolation) and 1.7 and 1.65 (CP6).  Corrected rows instead of swept ones, and constants
+    rounded once more, made it 1.74 and 1.26, 1.76 and 1.7."""
+    L = np.longdouble
+    cfg = C.channel(nc=(n, 16, 16), iacc=acc)
+    g = S.Solver(cfg)
+    for fam in (2, 3, 4, 5):
+        f = np.random.default_rng(n + fam).standard_normal((16, 16, n))
+        got = g.op3d(0, fam, (1, 1), f, None)
+        p = S.plan_inspect(cfg, 0, fam, (1, 1), False)
+        at = [np.roll(f.astype(L), -o, axis=2) for o in p["off"]]
+        r = (L(p["r1"]) * (at[0] + L(p["sgn"]) * at[1]) + L(p["r2"]) * (at[2] + L(p["sgn"]) * at[3])) * L(p["dd"])
+        # the left-hand side's off-diagonal is the plan's a
+        w = 1 + 2 * L(p["a"][3]) * np.cos(2 * L(np.pi) * np.arange(n // 2 + 1).astype(L) / n)
+        ref = sf.irfft(sf.rfft(r, axis=2) / w, n=n, axis=2)
+        err = np.linalg.norm((got - ref).astype(float)) / np.linalg.norm(ref.astype(float))
+        assert err <= bound[fam > 3] * 2.0 ** -53, (fam, err * 2.0 ** 53)
     g.close()
