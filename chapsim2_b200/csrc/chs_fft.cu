@@ -220,7 +220,7 @@ __device__ __forceinline__ void copy_twiddles(const FftPlan& fp, C* tw) {
 
 // strided lines, 1 << lsh of them per CTA
 template <typename C>
-__global__ void __launch_bounds__(512, 2) cfft_lines_kernel(const __grid_constant__ FftPlan fp, C* __restrict__ data,
+__global__ void __launch_bounds__(512, 2) cfft_lines_kernel(const __grid_constant__ FftPlan fp, C* data,
                                                             int na, int nlines, int64_t bstride, int64_t stride,
                                                             int sign, int lsh) {
   extern __shared__ __align__(16) unsigned char fft_smem[];
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(512, 2) rfft_rows_kernel(const __grid_constant
 }
 
 template <typename R, typename C>
-__global__ void __launch_bounds__(512, 2) irfft_rows_kernel(const __grid_constant__ FftPlan fp, const C* __restrict__ in,
+__global__ void __launch_bounds__(512, 2) irfft_rows_kernel(const __grid_constant__ FftPlan fp, const C* in,
                                                             R* __restrict__ out, int nrows, double scale, int pairs) {
   using S = typename Sc<C>::S;
   extern __shared__ __align__(16) unsigned char fft_smem[];

@@ -1158,7 +1158,7 @@ constexpr int kYsWarps = 16;
 
 template <typename C, int R>
 __global__ void __launch_bounds__(kYsWarps * 32, R == 8 ? 2 : 1)
-    ysolve_kernel(C* __restrict__ data, int nxh, int ny, int nz, const double* __restrict__ Zr,
+    ysolve_kernel(C* data, int nxh, int ny, int nz, const double* __restrict__ Zr,
                   const double* __restrict__ D, const double* __restrict__ pa) {
   using S = typename RealOf<C>::S;
   __shared__ double sE[kYsWarps][32], sM[kYsWarps][32];  // ends of the pieces, products of their multipliers
@@ -1239,7 +1239,7 @@ __global__ void __launch_bounds__(kYsWarps * 32, R == 8 ? 2 : 1)
 // arithmetic and its order are those of ysolve_kernel.
 constexpr int kYsBatch = 8;
 template <typename C>
-__global__ void __launch_bounds__(128) ysolve_lines_kernel(C* __restrict__ data, int nxh, int ny, int nz,
+__global__ void __launch_bounds__(128) ysolve_lines_kernel(C* data, int nxh, int ny, int nz,
                                                            const double* __restrict__ Zr,
                                                            const double* __restrict__ D,
                                                            const double* __restrict__ pa) {
@@ -1333,7 +1333,7 @@ template void launch_ysolve<double2>(double2*, int, int, int, const double*, con
 template void launch_ysolve<float2>(float2*, int, int, int, const double*, const double*, const double*,
                                     cudaStream_t, bool);
 
-__global__ void spectral_divide_kernel(double2* __restrict__ data, int nxh, int ny, int nz,
+__global__ void spectral_divide_kernel(double2* data, int nxh, int ny, int nz,
                                        const double* __restrict__ k2x, const double* __restrict__ k2y,
                                        const double* __restrict__ k2z, double norm) {
   grid_dep_launch();

@@ -142,6 +142,8 @@ void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstri
 // Chained launches: a kernel that calls grid_dep_wait() before it touches what its predecessor in the stream wrote, and
 // whose predecessor calls grid_dep_launch() early, may be launched with `chained`, so that its CTAs are set up
 // while the predecessor drains (programmatic dependent launch).  Not behind an event or as a graph's first node.
+// What the predecessor wrote is reached through plain pointers only: const __restrict__ and __ldg allow non-coherent
+// loads, and loads through a __restrict__ pointer may be moved above the wait.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
