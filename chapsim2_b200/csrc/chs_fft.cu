@@ -353,11 +353,6 @@ int row_pairs(const FftPlan& fp, int npairs) {
   return p;
 }
 
-template <typename K>
-void allow_smem(K kernel, size_t shm) {
-  if (shm > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-}
-
 }  // namespace
 
 void fft_stages(FftPlan& fp) {
@@ -398,7 +393,7 @@ template <typename R, typename C>
 void launch_rfft_rows(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream_t st) {
   const int npairs = (nrows + 1) / 2, pairs = row_pairs(fp, npairs), n = fp.n;
   const size_t shm = ((size_t)n + (size_t)pairs * (n + n / 8 + 1)) * sizeof(C);
-  allow_smem(rfft_rows_kernel<R, C>, shm);
+  allow_smem<rfft_rows_kernel<R, C>>(shm);
   rfft_rows_kernel<R, C><<<(npairs + pairs - 1) / pairs, fft_threads(fp, pairs, true), shm, st>>>(fp, in, out, nrows,
                                                                                                   pairs);
 }
@@ -406,7 +401,7 @@ template <typename R, typename C>
 void launch_irfft_rows(const FftPlan& fp, const C* in, R* out, int nrows, double scale, cudaStream_t st, bool chained) {
   const int npairs = (nrows + 1) / 2, pairs = row_pairs(fp, npairs), n = fp.n;
   const size_t shm = ((size_t)n + (size_t)pairs * (n + n / 8 + 1)) * sizeof(C);
-  allow_smem(irfft_rows_kernel<R, C>, shm);
+  allow_smem<irfft_rows_kernel<R, C>>(shm);
   launch_chained(irfft_rows_kernel<R, C>, dim3((npairs + pairs - 1) / pairs), dim3(fft_threads(fp, pairs, false)), shm,
                  st, chained, fp, in, out, nrows, scale, pairs);
 }
@@ -419,7 +414,7 @@ void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstri
   int lsh = sizeof(C) == 16 ? 4 : 5;
   while (lsh > 2 && (((size_t)fp.n << lsh) * sizeof(C) > 64 * 1024 || fft_threads(fp, 1 << lsh, false) > 512)) --lsh;
   const size_t shm = ((size_t)fp.n + ((size_t)fp.n << lsh)) * sizeof(C);
-  allow_smem(cfft_lines_kernel<C>, shm);
+  allow_smem<cfft_lines_kernel<C>>(shm);
   launch_chained(cfft_lines_kernel<C>, dim3((unsigned)((nlines + (1 << lsh) - 1) >> lsh)),
                  dim3(fft_threads(fp, 1 << lsh, false)), shm, st, chained, fp, data, na, (int)nlines, bstride, stride, sign,
                  lsh);

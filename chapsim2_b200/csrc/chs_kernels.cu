@@ -709,12 +709,7 @@ static void launch_dir(const OpPlan& P, const LineIOT<T>& io, const double* tabl
   switch (P.fam) {
 #define CHS_CASE(F)                                                                                   \
   case F: {                                                                                           \
-    static bool attr_set = false;                                                                     \
-    if (!attr_set) {                                                                                  \
-      cudaFuncSetAttribute(line_op_kernel<T, DIR, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                           kLineSmemMax);                                                             \
-      attr_set = true;                                                                                \
-    }                                                                                                 \
+    allow_smem<line_op_kernel<T, DIR, F>>(shm);                                                       \
     line_op_kernel<T, DIR, F><<<grid, block, shm, st>>>(P, io, table, nlines, LT);                    \
     break;                                                                                            \
   }
@@ -1055,7 +1050,7 @@ void launch_rfft_x(const FftPlan& fp, const R* in, C* out, int nrows, cudaStream
   const int lpc = fft_lines_per_cta(fp.n);
   const int npairs = (nrows + 1) / 2;
   const size_t shm = 2 * (size_t)lpc * fp.n * sizeof(C);
-  cudaFuncSetAttribute(rfft_x_kernel<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  allow_smem<rfft_x_kernel<R, C>>(shm);
   rfft_x_kernel<R, C><<<(npairs + lpc - 1) / lpc, 256, shm, st>>>(fp, in, out, nrows, lpc);
 }
 
@@ -1065,7 +1060,7 @@ void launch_irfft_x(const FftPlan& fp, const C* in, R* out, int nrows, double sc
   const int lpc = fft_lines_per_cta(fp.n);
   const int npairs = (nrows + 1) / 2;
   const size_t shm = 2 * (size_t)lpc * fp.n * sizeof(C);
-  cudaFuncSetAttribute(irfft_x_kernel<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  allow_smem<irfft_x_kernel<R, C>>(shm);
   irfft_x_kernel<R, C><<<(npairs + lpc - 1) / lpc, 256, shm, st>>>(fp, in, out, nrows, scale, lpc);
 }
 template void launch_rfft_x<double, double2>(const FftPlan&, const double*, double2*, int, cudaStream_t);
@@ -1082,7 +1077,7 @@ void launch_cfft_axis(const FftPlan& fp, C* data, int na, int nb, int64_t bstrid
   const int lpc = fft_lines_per_cta(fp.n);
   const int64_t nlines = (int64_t)na * nb;
   const size_t shm = 2 * (size_t)lpc * (fp.n + 1) * sizeof(C);
-  cudaFuncSetAttribute(cfft_axis_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  allow_smem<cfft_axis_kernel<C>>(shm);
   cfft_axis_kernel<C><<<(unsigned)((nlines + lpc - 1) / lpc), 256, shm, st>>>(fp, data, na, nb, bstride, stride,
                                                                                sign, lpc);
 }
@@ -1659,10 +1654,10 @@ void launch_dct_y(const FftPlan& fp, double2* data, int nxh, int nz, const doubl
   const unsigned grid = (unsigned)((nlines + lpc - 1) / lpc);
   if (ptab) {
     if (!pfac) throw std::runtime_error("dct_y: the pentadiagonal factors are missing");
-    cudaFuncSetAttribute(dct_y_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    allow_smem<dct_y_kernel<1>>(shm);
     dct_y_kernel<1><<<grid, 256, shm, st>>>(fp, data, nxh, nz, lpc, ayby, k2x, k2z, k2y, ptab, pfac, scale);
   } else {
-    cudaFuncSetAttribute(dct_y_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    allow_smem<dct_y_kernel<0>>(shm);
     dct_y_kernel<0><<<grid, 256, shm, st>>>(fp, data, nxh, nz, lpc, ayby, k2x, k2z, k2y, ptab, pfac, scale);
   }
 }

@@ -139,6 +139,18 @@ template <typename C>
 void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstride, int64_t stride, int sign,
                        cudaStream_t st, bool chained);
 
+// Dynamic shared memory above 48 KB is allowed per kernel, not per launch: always up to what the SM has beside the
+// kernel's static share, so that a handle of another size, perhaps in another thread, cannot lower it under a launch.
+template <auto K>
+inline void allow_smem(size_t shm) {
+  static const int limit = [] {
+    cudaFuncAttributes a{};
+    cudaFuncGetAttributes(&a, K);
+    return 227 * 1024 - (int)a.sharedSizeBytes;
+  }();
+  if (shm > 48 * 1024) cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
 // Chained launches: a kernel that calls grid_dep_wait() before it touches what its predecessor in the stream wrote, and
 // whose predecessor calls grid_dep_launch() early, may be launched with `chained`, so that its CTAs are set up
 // while the predecessor drains (programmatic dependent launch).  Not behind an event or as a graph's first node.

@@ -331,8 +331,7 @@ void launch_chunk(const OpPlan& P, const LineIOT<T>& io, const T* tab, cudaStrea
   const int W = (nmax + R - 1) / R;
   size_t shm = (size_t)(2 * W * 32 + 64 + 2 * W) * sizeof(T);
   if (DIR == 0) shm += (size_t)32 * (nmax | 1) * sizeof(T);
-  if (shm > 48 * 1024)
-    cudaFuncSetAttribute(line_chunk_kernel<T, DIR, CIN, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  allow_smem<line_chunk_kernel<T, DIR, CIN, R>>(shm);
   line_chunk_kernel<T, DIR, CIN, R><<<(nlines + 31) / 32, W * 32, shm, st>>>(P, io, tab, nlines);
 }
 
