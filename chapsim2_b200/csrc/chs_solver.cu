@@ -2739,7 +2739,9 @@ int chs_autotune(chs_handle* H, int nsteps, int* block, int* lt_max, int* fused,
     snapshot(H, snap, true);
     // 0: the specialised explicit-operator kernels; 128/256/512: the generic kernel's CTA size
     const int blocks[4] = {0, 128, 256, 512};
-    const bool compact = H->iacc >= 3;
+    // lines per CTA matter to compact lines without a form in register pieces only (more than 384 points)
+    bool tiles = false;
+    for (const auto& kv : H->plans) tiles = tiles || (kv.second.tdma && !kv.second.lrows);
     const int lts[3] = {16, 32, 64};
     int bb = 0, bl = 64, bf = 0;
     float best = 1e30f;
@@ -2747,7 +2749,7 @@ int chs_autotune(chs_handle* H, int nsteps, int* block, int* lt_max, int* fused,
       for (int fu = 0; fu <= 1; ++fu)
         for (int b : blocks)
           for (int l : lts) {
-            if (!compact && l != 64) continue;
+            if (!tiles && l != 64) continue;
             H->tune_block = b;
             H->tune_lt = l;
             H->tune_fuse = fu;

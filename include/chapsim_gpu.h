@@ -264,7 +264,8 @@ int chs_ensemble_destroy(chs_ensemble* e);
 
 /* Autotuner: times nsteps RK3 steps for each candidate launch shape (explicit
  * line operators: the specialised kernels, block 0, or the generic kernel with
- * a CTA size of 128/256/512; lines per CTA of the compact-scheme tile;
+ * a CTA size of 128/256/512; lines per CTA of
+ * the compact-scheme tile, which lines of more than 384 points take;
  * separate operators or fused per-component sums) on this handle, restoring
  * the state after each trial, and keeps the fastest. */
 int chs_autotune(chs_handle* h, int nsteps, int* block, int* lt_max, int* fused, float* best_ms);

@@ -42,6 +42,19 @@ def test_ensemble_matches_members_stepped_alone(precision):
         m.close()
 
 
+@pytest.mark.parametrize("nx", [16, 432])
+def test_autotune_lines_per_cta(nx):
+    """Lines per CTA are tried only where a compact line runs the tile kernel (more than 384 points); elsewhere the default
+    comes back every time and not whichever of three equal runs was quickest."""
+    cfg = C.channel(nc=(nx, 16, 12), iacc=C.IACCU_CP6, dt=1e-3)
+    g = S.Solver(cfg)
+    g.set_fields(*I.channel_fields(cfg))
+    g.Solve_momentum_eq(0)
+    got = {g.autotune(nsteps=1)[1] for _ in range(4 if nx == 16 else 1)}
+    assert got <= ({64} if nx == 16 else {16, 32, 64})
+    g.close()
+
+
 def test_autotune_keeps_the_state():
     cfg = C.channel(nc=(32, 24, 16), iacc=3, dt=0.004)
     f = I.channel_fields(cfg)
