@@ -1,11 +1,16 @@
 // FFTs of the Poisson solvers in at most three stages held in registers.
 //
-// A length n = 2^a 3^b up to 729 factors into at most three radices of 2, 3, 4, 6, 8, 9 (fft_stages), the largest in the middle.  The first Stockham stage takes its inputs from global memory and
-// the last stores its results there, so a line passes through shared memory once per stage boundary (twice
-// at most); the middle stage works in place, one butterfly per thread between two barriers.  The tile
-// has the lines side by side (z and y lines, whose 16 or 32 neighbouring columns are one 256-byte
-// segment of every row) or the positions padded by one in nine (x rows), which leaves every access of a
-// stage free of bank conflicts; twiddles are read from a copy in shared memory.
+// A length n = 2^a 3^b up to 729 factors into at most three radices of 2, 3, 4, 6, 8, 9 (fft_stages), the largest in
+// the middle.  The first Stockham stage takes its inputs from global memory and the last stores its results there, so a
+// line passes through shared memory once per stage boundary, twice at most; the middle stage works in place, one
+// butterfly per thread between two barriers.  The forward transform of real rows, whose spectra are formed from two
+// positions each, passes once more.  Twiddles are read from a copy in shared memory.
+//
+// z and y lines lie side by side in the tile, as many as 64 KB and 512 threads allow: segments of 256 bytes in every
+// row up to 256 points in FP64 (216: 128) and up to 128 in FP32 (108 and above 128: 128, above 256: 64), narrower
+// beyond.
+// Their accesses are free of bank conflicts from 8 lines (FP64) or 16 (FP32) up.  x rows are padded by one position in
+// nine, which keeps the stores of a first radix 2, 4 or 8 apart; 3, 6 and 9 meet in pairs.
 //
 // The kernels of chs_kernels.cu (radix 4, 2, 3 stages through two shared buffers with twiddles from
 // global memory) pass a line through shared memory nst + 1 times; they keep longer lines.  The four transforms of a
@@ -55,8 +60,8 @@ __device__ __forceinline__ C rot(C a, S c, S s) { return mk<C>(a.x * c - a.y * s
 template <typename C, typename S>
 __device__ __forceinline__ C rot90(C a, S sg) { return mk<C>(-sg * a.y, sg * a.x); }
 
-// x c for an irrational c = hi + lo.  A constant rounded once errs the same way in every product of every stage, forward
-// and back: with hi alone the FP64 solve of a 64^3 box errs by 4.2 units of 2^-53, with both by 3.5
+// x c for an irrational c = hi + lo.  A constant rounded once errs the same way in every product of every stage,
+// forward and back: with hi alone the FP64 solve of a 64^3 box errs by 4.2 units of 2^-53, with both by 3.5
 template <typename S>
 __device__ __forceinline__ S times(S x, S hi, S lo) { return fma(x, hi, x * lo); }
 template <typename S>
@@ -416,8 +421,8 @@ void launch_cfft_lines(const FftPlan& fp, C* data, int na, int nb, int64_t bstri
   const size_t shm = ((size_t)fp.n + ((size_t)fp.n << lsh)) * sizeof(C);
   allow_smem<cfft_lines_kernel<C>>(shm);
   launch_chained(cfft_lines_kernel<C>, dim3((unsigned)((nlines + (1 << lsh) - 1) >> lsh)),
-                 dim3(fft_threads(fp, 1 << lsh, false)), shm, st, chained, fp, data, na, (int)nlines, bstride, stride, sign,
-                 lsh);
+                 dim3(fft_threads(fp, 1 << lsh, false)), shm, st, chained, fp, data, na, (int)nlines, bstride, stride,
+                 sign, lsh);
 }
 template void launch_rfft_rows<double, double2>(const FftPlan&, const double*, double2*, int, cudaStream_t);
 template void launch_rfft_rows<float, double2>(const FftPlan&, const float*, double2*, int, cudaStream_t);

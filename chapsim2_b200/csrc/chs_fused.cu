@@ -622,8 +622,9 @@ __device__ __forceinline__ Pack<T, V> fz_row_v(const FzRow* __restrict__ rows, c
 }
 
 // ---- pressure update, projection and q = g / rho_face: V neighbours along x per thread, (i, j, k), j over the y
-// points.  Bound by its streams (13 fields with variable properties); with one value per thread the index work of the
-// loads filled 77 % of the issue slots at 43 % of the memory rate in FP32 (384x256x384: 456 us with one, 397 with two).
+// points.  Bound by its streams (13 fields with variable properties): 44 % of the memory rate in FP64 at 128x96x128.  One
+// value per thread spends its issue slots on the index work of the loads (384x256x384 FP32: 456 us with one, 397 with
+// two).
 template <typename T, bool TH, int V>
 __global__ void __launch_bounds__(256) fz_project_kernel(const __grid_constant__ FzProject<T> f) {
   using W = Pack<T, V>;
@@ -863,10 +864,12 @@ void launch_fz_project(const FzProject<T>& f, cudaStream_t st, bool chained) {
   dim3 bs, grid;
   if (f.n0 % 2 == 0) {
     pack_shape(f.n0 / 2, f.np1, f.n2, bs, grid);
-    launch_chained(f.thermo ? fz_project_kernel<T, true, 2> : fz_project_kernel<T, false, 2>, grid, bs, 0, st, chained, f);
+    launch_chained(f.thermo ? fz_project_kernel<T, true, 2> : fz_project_kernel<T, false, 2>, grid, bs, 0, st, chained,
+                   f);
   } else {
     pack_shape(f.n0, f.np1, f.n2, bs, grid);
-    launch_chained(f.thermo ? fz_project_kernel<T, true, 1> : fz_project_kernel<T, false, 1>, grid, bs, 0, st, chained, f);
+    launch_chained(f.thermo ? fz_project_kernel<T, true, 1> : fz_project_kernel<T, false, 1>, grid, bs, 0, st, chained,
+                   f);
   }
 }
 

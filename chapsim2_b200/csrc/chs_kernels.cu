@@ -1091,7 +1091,7 @@ template void launch_cfft_axis<float2>(const FftPlan&, float2*, int, int, int64_
 // The forward-sweep factors of TRID0 depend only on (kx, kz), not on the right-hand side, so
 // they are computed once: Zr[j] = 1/pivot_j (j < ny-1), D[j] = c_j * Zr[j], and for the last
 // row the pivot itself, or 0 when it is pinned (|pivot| <= 1e-10).  Layout (kz, j, kx) like the
-// spectrum.  The arithmetic is TRID0's, in its order, so the solve is bitwise the same.
+// spectrum.  The factors' arithmetic is TRID0's, in its order.
 __global__ void ysolve_factor_kernel(double* __restrict__ Zr, double* __restrict__ D, int nxh, int ny, int nz,
                                      const double* __restrict__ pa, const double* __restrict__ pb,
                                      const double* __restrict__ pc, const double* __restrict__ lamx,
@@ -1140,7 +1140,9 @@ __device__ __forceinline__ float2 from_d2<float2>(double2 v) { return make_float
 // Columns of up to 160 rows: a CTA owns 16 consecutive columns, lane 2 l + part the real or imaginary part
 // of column l (the system is real), warp w rows w R .. w R + R - 1, all in registers.  A piece is swept twice in
 // each direction: from zero, for its end value and the product of its multipliers, then, once the value
-// entering it is known from the pieces before it, with TRID0's recurrences from that value.  One
+// entering it is known from the pieces before it, from that value.  The rows are scaled by their pivots'
+// reciprocals first, the last one too; against TRID0's order of operations that changes the error of a solve by less
+// than its spread over right-hand sides (1.4e-14 to 1.6e-13 of the pressure on five grids).  One
 // thread per column swept the tile it replaces from shared memory (16 of 128 threads busy); the whole
 // solve in flight instead takes FP64 128x96x128 from 16.5 to 12.4 us, with an FP32 spectrum to 10.4.
 template <typename C>
@@ -1231,7 +1233,7 @@ __global__ void __launch_bounds__(kYsWarps * 32, R == 8 ? 2 : 1)
 // The same solve with one thread per (kx, kz) line working in place in global memory: at a fixed
 // row j the threads of a warp (consecutive kx) read and write consecutive values, and each thread
 // loads eight rows ahead of its sweep, so the sequential recurrences of many lines overlap.  The
-// arithmetic and its order are those of ysolve_kernel.
+// arithmetic and its order are TRID0's.
 constexpr int kYsBatch = 8;
 template <typename C>
 __global__ void __launch_bounds__(128) ysolve_lines_kernel(C* data, int nxh, int ny, int nz,
@@ -1312,11 +1314,13 @@ void launch_ysolve(C* data, int nxh, int ny, int nz, const double* Zr, const dou
                    cudaStream_t st, bool chained) {
   if (ny < 2) throw std::runtime_error("ysolve: ny must be at least 2");
   const int64_t n = (int64_t)nxh * nz;
-  // 16 rows a thread at 256 rows: 191 us at 384x256x384 in FP32 against 176 by the lines kernel
+  // Rows in pieces up to 160, where the shared-memory tile that the pieces replaced ended.  Measured in us, FP64 and with
+  // an FP32 spectrum, by lines / pieces / the tile: 128x144x128 38 / 21 / 40 and 45 / 19 / 41, 384x160x384 147 / 211 / 334
+  // and 105 / 164 / 425; above 160 rows by lines / pieces: 128x256x128 64 / 29 and 77 / 25, 384x256x384 FP32 176 / 191.
   const int R = ny <= 8 * kYsWarps ? 8 : 16;
   if (ny > 160) {
-    launch_chained(ysolve_lines_kernel<C>, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, st, chained, data, nxh, ny, nz,
-                   Zr, D, pa);
+    launch_chained(ysolve_lines_kernel<C>, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, st, chained, data, nxh, ny,
+                   nz, Zr, D, pa);
     return;
   }
   const unsigned blocks = (unsigned)((n + 15) / 16), threads = (unsigned)((ny + R - 1) / R * 32);
@@ -1351,7 +1355,8 @@ __global__ void spectral_divide_kernel(double2* data, int nxh, int ny, int nz,
 
 void launch_spectral_divide(double2* data, int nxh, int ny, int nz, const double* k2x, const double* k2y,
                             const double* k2z, double norm, cudaStream_t st, bool chained) {
-  launch_chained(spectral_divide_kernel, dim3(148 * 8), dim3(256), 0, st, chained, data, nxh, ny, nz, k2x, k2y, k2z, norm);
+  launch_chained(spectral_divide_kernel, dim3(148 * 8), dim3(256), 0, st, chained, data, nxh, ny, nz, k2x, k2y, k2z,
+                 norm);
 }
 
 // ===========================================================================

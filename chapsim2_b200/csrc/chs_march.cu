@@ -14,7 +14,9 @@
 // component through L1 at 64 registers, 22-34 % of the memory rate.  Here a cell's inputs are loaded
 // once (1.4x with the halo), and the history and output streams are the only other traffic.  Per substep, the
 // three components then and the march now: 128x96x128 heated FP64 150 and 64 us, 384x256x384 heated FP32 2700 and
-// 837 us (3.1 TB/s).  FP64 runs 20 warps per SM (96 registers); FP32 30, bound by shared-memory reads and barriers.
+// 837 us (3.1 TB/s).  FP64 runs 20 warps per SM (96 registers) and waits between the two barriers of a plane: 47 % of the
+// issue slots, 56 % of the shared-memory wavefronts, 34 % of the memory rate at 128x96x128.  FP32 runs 30 and fills 66 %
+// of the issue slots at the same shared-memory share.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -116,7 +118,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3)
       if (e < Sz::pairs) {
         const unsigned kind = kinds >> (2 * u) & 3u;
         if (kind == 2u || !z_only)
-          copy_pair(set + 2 * e, from[u * kThreads + threadIdx.x] + (kind == 0u ? off_c : (kind == 1u ? off_y : off_z)));
+          copy_pair(set + 2 * e,
+                    from[u * kThreads + threadIdx.x] + (kind == 0u ? off_c : (kind == 1u ? off_y : off_z)));
       }
     }
     if (wall_from && !z_only) copy_pair(set + kData + 2 * threadIdx.x, wall_from + kw * n0);

@@ -1386,8 +1386,10 @@ bool fz_march_form(const chs_handle* H, const FzMomentum<T>& F) {
   return per(F.pres[0], dx) && c2p(F.pres[1], true, false) && per(F.pres[2], dz);
 }
 
-// Momentum right-hand sides, fractional step, mass-flux mean and advance of the substep in four
-// launches (wall planes, fused momentum, mean, advance) instead of the ~50 of the operator path.
+// Momentum right-hand sides, fractional step and mass-flux mean of the substep instead of the ~50 launches of the
+// operator path: the y walls' planes, then the march (with the y component's wall rows beside it) or, where its
+// operators are not the march's, a pass per component and one for the mean.  Unless the advance is deferred to the
+// Poisson right-hand side and the projection, a last launch makes it.
 // Returns false (nothing launched) when the configuration needs the operator path.
 template <typename T>
 bool fused_momentum(chs_handle* H, int isub, double* ux, double* uy, double* uz, bool defer_update) {
@@ -1738,8 +1740,9 @@ void substep_body_t(chs_handle* H, int isub, int parts) {
   double* uz = TH ? H->gz : H->qz;
 
   const int w0 = B[1][V_QY][0] == BC_DIRICHLET, w1 = B[1][V_QY][1] == BC_DIRICHLET;
-  // fused path: the momentum advance u += m - bulk is not stored by itself but formed where the
-  // Poisson right-hand side and the projection read u (both fused kernels must be available)
+  // fused path: the advanced fields are stored by the momentum pass (x, whose mass-flux mean is known only after it, as
+  // its increment), and the mean is taken off where the Poisson right-hand side and the projection read them; u itself
+  // is written by the projection only (both fused kernels must be available)
   FzUpdateDiv<T> F{};
   const bool defer = fused_div_form<T>(H, isub, ux, w0, w1, F) &&
                      fused_project<T>(H, isub, ux, uy, uz, w0, w1, true, false);
@@ -2151,7 +2154,9 @@ void thermo_init(chs_handle* H, const chs_thermo* c) {
   std::vector<double2> pairs(7 * (size_t)n, make_double2(0.0, 0.0));
   for (int i = 0; i < n; ++i) {
     // the last row starts no interval
-    auto slope = [&](const double* y, const double* x) { return i + 1 < n ? (y[i + 1] - y[i]) / (x[i + 1] - x[i]) : 0.0; };
+    auto slope = [&](const double* y, const double* x) {
+      return i + 1 < n ? (y[i + 1] - y[i]) / (x[i + 1] - x[i]) : 0.0;
+    };
     pairs[2 * i] = make_double2(rhoh[i], c->h[i]);
     pairs[2 * i + 1].x = slope(c->h, rhoh.data());
     double2* r = pairs.data() + 2 * (size_t)n + 5 * (size_t)i;
@@ -2611,7 +2616,8 @@ void run_step(chs_handle* H) {
 }
 
 void capture_graphs(chs_handle* H) {
-  for (int isub = 1; isub <= 3; ++isub) H->kernels_per_sub[isub] = capture_one(H, isub, isub, PART_ALL, &H->gexec[isub]);
+  for (int isub = 1; isub <= 3; ++isub)
+    H->kernels_per_sub[isub] = capture_one(H, isub, isub, PART_ALL, &H->gexec[isub]);
 }
 
 void capture_part_graphs(chs_handle* H) {
