@@ -1,29 +1,29 @@
 // Compact line operators with the line kept in registers (CP4 and CP6).
 //
-// A CTA owns 32 lines.  Warp w holds rows w*R .. w*R + R-1 of every one of them, lane l those of line
-// l, so a thread solves a piece of R rows of one line.  Each direction of the Thomas sweep
+// A CTA owns 32 lines.  Warp w holds rows w*R .. w*R + R-1 of every one of them, lane l those of line l, so a
+// thread solves a piece of R rows of one line.  Each direction of the Thomas sweep
 //
 //   forward   y_i = (r_i - a_i y_{i-1}) D_i       backward   x_i = y_i - C_i x_{i+1}
 //
-// with D = 1/pivot and C = c/pivot (line_coefs in chs_plan.cpp) runs over a piece twice: from zero, for the value at
-// the piece's end, and, once the value entering the piece is known, from that value.  It follows from the ends of the
-// pieces before: end of a piece = its end from zero + (product of its -a D, or -C) times the value entering it, over at
-// most 16 pieces, which each thread runs for itself from shared memory.  The last row of a periodic line stands
-// outside the Thomas system (its row of factors passes the right-hand side through) and closes it as
-// Solve_TDMA_cyclic does (src/basics_algorithms.f90:60-109).
+// with D = 1/pivot and C = c/pivot (line_coefs in chs_plan.cpp) needs the value entering the piece.  It follows
+// from the ends of the pieces before: end of a piece = its end for a sweep from zero + (product of its -a D, or
+// -C) times the value entering it, over at most 16 pieces, which each thread runs for itself from shared memory.
+// The end for a sweep from zero is a weighted sum of the piece's rows (host tables): no chain, half the products
+// of a sweep.  The last row of a periodic line stands outside the Thomas system (its row of factors passes the
+// right-hand side through) and closes it as Solve_TDMA_cyclic does (src/basics_algorithms.f90:60-109).
 //
-// The second sweep instead of a correction of every row, y_i += P_i y_in, keeps the rounding of the plain sweep: the
-// corrected rows, with r1 dd and a D as one constant each, erred by up to 1.34 times as much (CP4 differences at 128
-// points, 1.74 and 1.28 units of 2^-53; FP32 velocities of a CP6 channel 4 to 9 % more).
+// Sweeping the rows from the value that enters, and not correcting rows swept from zero (y_i += P_i y_in), keeps
+// the rounding of the plain sweep: the corrected rows, with r1 dd and a D as one constant each, erred by up to
+// 1.34 times as much (CP4 differences at 128 points, 1.74 and 1.28 units of 2^-53; FP32 velocities of a CP6
+// channel 4 to 9 % more).
 //
-// What bounds it: with one thread per line (line_op_kernel) a CTA ran two sweeps of n dependent rows
-// in one warp of eight while the others waited, and reached 15 % of the memory rate.  Here every warp
-// sweeps R rows, all R + 3 input values of a thread are in flight at once, and for y and z lines
-// neither input nor output passes through shared memory (32 neighbouring x positions are one 256-byte
-// segment of FP64 at every row); x lines are transposed through a shared tile with an odd stride.
-// Pieces of 8 rows beat 16 (shorter chains, twice the warps): FP64 line solves of a substep, one sweep and a
-// correction, 128x96x128 CP6 channel 486 against 593 us (1029 us by line_op_kernel), Taylor-Green 96^3 244 against
-// 322 us.  With the second sweep 502 and 248 us.
+// What bounds it: with one thread per line (line_op_kernel) a CTA ran two sweeps of n dependent rows in one warp
+// of eight while the others waited, and reached 15 % of the memory rate.  Here every warp sweeps R rows, all R + 3
+// input values of a thread are in flight at once, and for y and z lines neither input nor output passes through
+// shared memory (32 neighbouring x positions are one 256-byte segment of FP64 at every row); x lines are
+// transposed through a shared tile with an odd stride.  Pieces of 8 rows beat 16 (shorter chains, twice the warps):
+// FP64 line solves of a substep of the 128x96x128 CP6 channel 479 us (corrected rows 484, of 16 rows 593;
+// line_op_kernel 1029), of the Taylor-Green 96^3 box 235 us (239, 322); with FP32 fields 355 and 350 us.
 #include <cuda_runtime.h>
 
 #include <stdexcept>
@@ -35,7 +35,7 @@ namespace chs {
 
 namespace {
 
-// the factors of one row (line_coefs): d, a | c, q | x, m | p, unused
+// the factors of one row (line_coefs): d, a | c, x | g, h | m, e
 template <typename T>
 struct Pair2;
 template <>
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
   // last two rows of a periodic line
   const bool edge = i0 + kLo < 0 || i0 + kLo + N > nin || i0 < P.b_lo || i0 + R - 1 > P.b_hi || i0 + R > nout - 2;
   if (threadIdx.x < W) {
-    sP[threadIdx.x] = coef2(tab, threadIdx.x * R + R - 1, 3).x;
-    sP[W + threadIdx.x] = coef2(tab, threadIdx.x * R, 1).y;
+    sP[threadIdx.x] = coef1(tab, threadIdx.x * R + R - 1, 7);
+    sP[W + threadIdx.x] = coef1(tab, threadIdx.x * R, 7);
   }
 
   int base = 0, obase = 0, ps = 1;  // first value of the line in the input and output, row stride
@@ -225,13 +225,11 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
   }
   // ---- end of the forward piece
   {
-    T y = T(0);
+    // the row that weighs most last, so that the sums before it round finer
+    T e[2] = {T(0), T(0)};
 #pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const auto da = coef2(tab, i0 + u, 0);
-      y = x[u] * da.x - (da.y * da.x) * y;
-    }
-    sE[w * 32 + lane] = y;
+    for (int u = 0; u < R - 1; ++u) e[u & 1] += coef1(tab, i0 + u, 4) * x[u];
+    sE[w * 32 + lane] = coef1(tab, i0 + R - 1, 4) * x[R - 1] + (e[0] + e[1]);
   }
   __syncthreads();
   // ---- forward sweep from the joined value, start of the backward piece
@@ -252,10 +250,10 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
         if (i0 + u == nout - 1) sN[32 + lane] = x[u];
       }
     }
-    T z = T(0);
+    T f[2] = {T(0), T(0)};
 #pragma unroll
-    for (int u = R - 1; u >= 0; --u) z = x[u] - coef1(tab, i0 + u, 2) * z;
-    sF[w * 32 + lane] = z;
+    for (int u = R - 1; u > 0; --u) f[u & 1] += coef1(tab, i0 + u, 5) * x[u];
+    sF[w * 32 + lane] = x[0] + (f[0] + f[1]);
   }
   __syncthreads();
   // ---- backward sweep from the joined value, cyclic closure, metric and wall slopes
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
     }
     if (P.tdma == 2) {
 #pragma unroll
-      for (int u = 0; u < R; ++u) x[u] += coef1(tab, i0 + u, 4) * xn;
+      for (int u = 0; u < R; ++u) x[u] += coef1(tab, i0 + u, 3) * xn;
     }
     if (edge && P.tdma == 2) {
 #pragma unroll
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(kLineWarps * 32, (R == 8 ? 2 : 1))
     }
     if (P.lmap >= 0) {
 #pragma unroll
-      for (int u = 0; u < R; ++u) x[u] *= coef1(tab, i0 + u, 5);
+      for (int u = 0; u < R; ++u) x[u] *= coef1(tab, i0 + u, 6);
     }
     if (edge && (P.neu1 || P.neu2)) {
 #pragma unroll

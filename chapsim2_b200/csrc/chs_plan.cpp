@@ -736,10 +736,11 @@ OpPlan PlanBook::make(int d, int fam, const int ibc0[2], bool has_fbc) {
   return p;
 }
 
-// Row factors of a compact line cut into pieces of lrows rows (chs_line.cu): D = 1/pivot, the sub-diagonal a,
-// C = c/pivot, Q the product of the -C to the piece's end, the cyclic correction X, the metric M, P the product
-// of the -a D from the piece's start.  Rows past the end are zero; the last row of a periodic line, which is not part of the
-// Thomas system, passes its right-hand side through.
+// Row factors of a compact line cut into pieces of lrows rows (chs_line.cu): D = 1/pivot, the sub-diagonal a, C =
+// c/pivot, the cyclic correction X, the weights G and H of the row in its piece's end value of a forward and a
+// backward sweep from zero, the metric M, and E: at a piece's last row the product of its -a D, at its first that
+// of its -C.  Rows past the end are zero; the last row of a periodic line, which is not part of the Thomas system,
+// passes its right-hand side through.
 void PlanBook::line_coefs(OpPlan& p) {
   const int n = p.nout, R = line_piece_rows(std::max(p.nin, p.nout));
   if (R == 0) return;
@@ -751,11 +752,22 @@ void PlanBook::line_coefs(OpPlan& p) {
     at(i, 0) = !in ? 1.0 : (i == 0 ? 1.0 / p.b1 : table[p.ld + i]);
     at(i, 1) = in && i > 0 ? table[p.la + i] : 0.0;
     at(i, 2) = i < nsw - 1 ? table[p.lc + i] : 0.0;
-    at(i, 4) = p.tdma == 2 && in ? table[p.lx1 + i] : 0.0;
-    at(i, 5) = p.lmap >= 0 ? table[p.lmap + i] : 1.0;
+    at(i, 3) = p.tdma == 2 && in ? table[p.lx1 + i] : 0.0;
+    at(i, 6) = p.lmap >= 0 ? table[p.lmap + i] : 1.0;
   }
-  for (int i = 0; i < rows; ++i) at(i, 6) = -at(i, 1) * at(i, 0) * (i % R == 0 ? 1.0 : at(i - 1, 6));
-  for (int i = rows - 1; i >= 0; --i) at(i, 3) = -at(i, 2) * (i % R == R - 1 ? 1.0 : at(i + 1, 3));
+  for (int i0 = 0; i0 < rows; i0 += R) {
+    double p = 1.0, q = 1.0;
+    for (int i = i0 + R - 1; i >= i0; --i) {
+      at(i, 4) = p * at(i, 0);
+      p *= -at(i, 1) * at(i, 0);
+    }
+    for (int i = i0; i < i0 + R; ++i) {
+      at(i, 5) = q;
+      q *= -at(i, 2);
+    }
+    at(i0 + R - 1, 7) = p;
+    at(i0, 7) = q;
+  }
   std::vector<float> f32(f.begin(), f.end());
   std::vector<double> packed(f.size() / 2);
   std::memcpy(packed.data(), f32.data(), f32.size() * sizeof(float));
